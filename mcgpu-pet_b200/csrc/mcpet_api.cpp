@@ -49,31 +49,6 @@ void dfree(T*& p) {
 constexpr int kMaxStepsDefault = 1 << 20;       /* Woodcock steps per photon */
 constexpr int kMaxRejectionsDefault = 1 << 16;  /* iterations per sampler rejection loop */
 
-/* (a^e) mod m with exact 64-bit arithmetic. */
-uint32_t powmod(uint64_t a, uint64_t e, uint64_t m) {
-  uint64_t r = 1 % m;
-  a %= m;
-  while (e) {
-    if (e & 1) r = (r * a) % m;
-    a = (a * a) % m;
-    e >>= 1;
-  }
-  return (uint32_t)r;
-}
-
-/* Powers (a^C)^(2^k) mod m for the stream jump, C = 555555*256 draws per
- * stream (the reference init_PRNG leap, MCGPU-PET_kernel.cu:251-253,925-978). */
-void jump_tables(int32_t* t1, int32_t* t2) {
-  const uint64_t C = (uint64_t)kLeapHistories * kLeapDistance;
-  uint64_t p1 = powmod(40014, C, 2147483563ull), p2 = powmod(40692, C, 2147483399ull);
-  for (int k = 0; k < 32; ++k) {
-    t1[k] = (int32_t)p1;
-    t2[k] = (int32_t)p2;
-    p1 = (p1 * p1) % 2147483563ull;
-    p2 = (p2 * p2) % 2147483399ull;
-  }
-}
-
 int pick_device(int requested) {
   int count = 0;
   if (cudaGetDeviceCount(&count) != cudaSuccess || count <= 0) return -1;
@@ -129,7 +104,6 @@ void fill_params(const mcpet_scene* sc, TransportParams& P) {
   P.span = c.span;
   P.nsinos = c.n_sinograms;
   P.nbins = c.n_bins;
-  jump_tables(P.jump1, P.jump2);
   P.seed = c.seed;
   int ms = 1;
   for (int m = 0; m < kMaxMaterials; ++m)
@@ -2271,7 +2245,6 @@ mcpet_status mcpet_probe_rng(int n, int seed_input, const int64_t* stream_ids, i
   if (s != MCPET_OK) return s;
   TransportParams P;
   memset(&P, 0, sizeof(P));
-  jump_tables(P.jump1, P.jump2);
   P.seed = seed_input;
   DBuf<int64_t> ids;
   DBuf<int2> sd;

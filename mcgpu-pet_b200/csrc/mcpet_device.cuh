@@ -73,27 +73,61 @@ __device__ __forceinline__ uint32_t mulmod_pm(uint32_t a, uint32_t b, uint32_t c
   return q >= m ? q - m : q;
 }
 
-/* Start state of RANECU stream `stream` for a seed: the reference
- * jumps each thread (stream+1)*555555*256 draws ahead
- * (init_PRNG, MCGPU-PET_kernel.cu:925-978).  a^((s+1)C) = prod over the set
- * bits of (s+1) of (a^C)^(2^k), with the 32 powers precomputed on the host. */
-__device__ __forceinline__ Rng rng_stream(const TransportParams& P, int seed, uint64_t stream) {
-  uint64_t e = stream + 1;
-  uint32_t y1 = 1, y2 = 1;
-#pragma unroll 4
-  for (int k = 0; k < 32; ++k) {
-    if ((e >> k) & 1ull) {
-      y1 = mulmod_pm(y1, (uint32_t)P.jump1[k], 85u, kM1);
-      y2 = mulmod_pm(y2, (uint32_t)P.jump2[k], 249u, kM2);
-    }
+/* Powers (a^C)^(v 256^w) mod m of both generators for every value v of the
+ * four bytes w of a stream number, C = 555555 * 256 draws a stream (the
+ * reference's leap, MCGPU-PET_kernel.cu:251-253, 925-978); 8 KB, evaluated by
+ * the compiler. */
+struct JumpTable {
+  uint2 power[4][256];
+};
+constexpr uint32_t constexpr_mulmod(uint32_t a, uint32_t b, uint32_t m) { return (uint32_t)((uint64_t)a * b % m); }
+constexpr uint32_t constexpr_powmod(uint32_t a, uint64_t e, uint32_t m) {
+  uint32_t r = 1;
+  for (; e; e >>= 1) {
+    if (e & 1) r = constexpr_mulmod(r, a, m);
+    a = constexpr_mulmod(a, a, m);
   }
-  Rng r;
-  r.x = (int)mulmod_pm((uint32_t)seed % kM1, y1, 85u, kM1);
-  r.y = (int)mulmod_pm((uint32_t)seed % kM2, y2, 249u, kM2);
   return r;
 }
-__device__ __forceinline__ Rng rng_stream(const TransportParams& P, uint64_t stream) {
-  return rng_stream(P, P.seed, stream);
+constexpr JumpTable make_jump_table() {
+  JumpTable t = {};
+  const uint64_t leap = (uint64_t)kLeapHistories * kLeapDistance;
+  uint32_t b1 = constexpr_powmod(40014, leap, kM1), b2 = constexpr_powmod(40692, leap, kM2);
+  for (int w = 0; w < 4; ++w) {
+    uint32_t p1 = 1, p2 = 1;
+    for (int v = 0; v < 256; ++v) {
+      t.power[w][v].x = p1;
+      t.power[w][v].y = p2;
+      p1 = constexpr_mulmod(p1, b1, kM1);
+      p2 = constexpr_mulmod(p2, b2, kM2);
+    }
+    b1 = p1;   /* (a^C)^(256^(w+1)) */
+    b2 = p2;
+  }
+  return t;
+}
+static __device__ const JumpTable kJump = make_jump_table();
+
+/* Start state of RANECU stream `stream` for a seed: the reference
+ * jumps each thread (stream+1)*555555*256 draws ahead
+ * (init_PRNG, MCGPU-PET_kernel.cu:925-978).  a^((s+1)C) is the product of one
+ * power for each byte of s+1: two modular products a byte, their four loads
+ * independent, where the bits of s+1 one by one cost up to 64 products (and a
+ * warp paid for the bits of all its lanes).  That start was most of a lane's
+ * work where lanes hold about one decay. */
+__device__ __forceinline__ Rng rng_stream(int seed, uint64_t stream) {
+  const uint32_t e = (uint32_t)(stream + 1);
+  uint2 y = __ldg(&kJump.power[0][e & 255u]);
+#pragma unroll
+  for (int w = 1; w < 4; ++w) {
+    const uint2 f = __ldg(&kJump.power[w][(e >> (8 * w)) & 255u]);
+    y.x = mulmod_pm(y.x, f.x, 85u, kM1);
+    y.y = mulmod_pm(y.y, f.y, 249u, kM2);
+  }
+  Rng r;
+  r.x = (int)mulmod_pm((uint32_t)seed % kM1, y.x, 85u, kM1);
+  r.y = (int)mulmod_pm((uint32_t)seed % kM2, y.y, 249u, kM2);
+  return r;
 }
 
 /* ------------------------------------------------------------------------

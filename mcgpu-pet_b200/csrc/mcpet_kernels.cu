@@ -32,7 +32,7 @@ __global__ void probe_rng_kernel(TransportParams P, int n, const int64_t* ids, i
                                  float* draws, double* ddraws) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  Rng r = rng_stream(P, (uint64_t)ids[i]);
+  Rng r = rng_stream(P.seed, (uint64_t)ids[i]);
   seeds[i] = make_int2(r.x, r.y);
   Rng r2 = r;
   for (int d = 0; d < ndraw; ++d) draws[(size_t)i * ndraw + d] = ranecu(r);

@@ -86,9 +86,6 @@ struct TransportParams {
   float e_resol, e_low, e_high, fovz;
   int nrows, ncrystals, nangles, nrad, nzs, ne, mrd, span, nsinos;
   long long nbins;
-  /* RANECU jump tables: (a^(555555*256))^(2^k) mod m, k = 0..31 */
-  int32_t jump1[32];
-  int32_t jump2[32];
   int seed;
   /* lane plan */
   uint64_t n_lanes;
