@@ -538,6 +538,24 @@ mcpet_status enqueue_run(mcpet_scene* sc, const mcpet_run_opts* opts, DeviceTall
   return launch_planned(sc, o, P, O, st, ms_out);
 }
 
+/* Decays of a scene's full acquisition (also while the autotuner runs it on
+ * a sample). */
+double scene_decays(const mcpet_scene* sc) {
+  return emitting_activity(sc) * ((double)sc->cfg.acquisition_time_ps * 1e-12) / sc->tune_scale;
+}
+
+/* Whether a launch of `decays` expected decays, at most `longest` of them in
+ * one lane, starts its longest lanes on warps of their own: where their
+ * chains bound the run.  A chain takes about 26 us a decay in a full warp
+ * (8 us alone) and the whole GPU 0.4 ns a decay, so the chains of a packed
+ * start end after the rest when a lane holds more than about 1/65000 of the
+ * decays; the line is at four times that, where spreading gains whatever the
+ * lanes share.  Above it a spread start is 3 times faster (1e7 decays of the
+ * 9^3 cube, a lane 1/330 of them: 773 -> 253 ms); below, packed lanes share
+ * voxels and scenes (58 095 decays of the cube, a lane 1/58095: 0.417 ms
+ * packed, 0.432 spread; the 1e9-decay head: equal). */
+int spread_lanes(double longest, double decays) { return longest * 16384.0 > decays ? 1 : 0; }
+
 /* Kernel variant of a run: balanced lanes use the single-precision
  * rotation and decay clock (they are held to statistical parity; reference
  * lanes keep the reference's arithmetic for replay), prompt-gamma scenes the
@@ -571,6 +589,7 @@ mcpet_status launch_planned(mcpet_scene* sc, const mcpet_run_opts& o, TransportP
       return set_error(MCPET_ERR_ARG, "lowered loop caps are not available for the gradient's recording run");
     if (algorithm != kAlgorithmEvents || (mode & kTransportPrompt)) algorithm = kAlgorithmHistories;
   }
+  P.spread_lanes = spread_lanes(d.max_lane_decays, scene_decays(sc));
   size_t smem = transport_dynamic_smem(P, block, algorithm);
   int bps = 0;
   CUDA_TRY(transport_occupancy(counters, algorithm, mode, block, smem, &bps));
@@ -837,12 +856,6 @@ struct BatchLaunch {
  * chained variant is the plain event kernel). */
 constexpr double kSoloDecays = 2.0e7;
 
-/* Decays of a scene's full acquisition (also while the autotuner runs it on
- * a sample). */
-double scene_decays(const mcpet_scene* sc) {
-  return emitting_activity(sc) * ((double)sc->cfg.acquisition_time_ps * 1e-12) / sc->tune_scale;
-}
-
 /* True when scene b has scene a's scanner: detector, sinogram, energy
  * window and tally settings, and the acquisition time of the PSF records
  * (every parameter detect_pair reads). */
@@ -955,9 +968,16 @@ mcpet_status setup_batch(mcpet_scene* const* scenes, int n, const mcpet_run_opts
       lanes += L.slots[(size_t)i].P.n_lanes;
     }
     L.total += lanes;
+    double longest = 0, decays = 0;
+    for (int i = j; i < j + g.count; ++i) {
+      const mcpet_scene* sc = scenes[L.scene_of[(size_t)i]];
+      longest = std::max(longest, sc->dev.max_lane_decays);
+      decays += scene_decays(sc);
+    }
     if (g.solo) {
       const int k = L.scene_of[(size_t)j];
       g.P = alone[(size_t)k];
+      g.P.spread_lanes = spread_lanes(longest, decays);
       g.T = L.slots[(size_t)j].T;
       g.O = L.slots[(size_t)j].O;
       g.mode = run_mode(scenes[k], o) | kTransportChained;
@@ -968,6 +988,7 @@ mcpet_status setup_batch(mcpet_scene* const* scenes, int n, const mcpet_run_opts
     }
     g.P = L.slots[(size_t)j].P;
     g.P.n_lanes = lanes;
+    g.P.spread_lanes = spread_lanes(longest, decays);
     g.P.n_emitters = 0;
     g.P.max_shells = max_shells;
     /* the launch's shared layout holds the prompt-gamma fields when any of
@@ -2043,8 +2064,8 @@ mcpet_status mcpet_run_psf_stream(mcpet_scene* sc, const mcpet_run_opts* opts, l
       R.mat_dose = nullptr;
       R.vox_dose = nullptr;
     }
-    unsigned long long begin = b;
-    CUDA_TRY(cudaMemcpyAsync(O.lane_cursor, &begin, sizeof(begin), cudaMemcpyHostToDevice, st));
+    Q.first_lane = b;
+    CUDA_TRY(cudaMemsetAsync(O.lane_cursor, 0, sizeof(unsigned long long), st));
     CUDA_TRY(cudaMemsetAsync(O.psf_count, 0, 4, st));
     double ms = 0;
     mcpet_status r = launch_planned(sc, o, Q, R, st, &ms);

@@ -88,7 +88,8 @@ struct TransportParams {
   long long nbins;
   int seed;
   /* lane plan */
-  uint64_t n_lanes;
+  uint64_t n_lanes;       /* end of the launch's lanes */
+  uint64_t first_lane;    /* their start (0 but for runs over ranges of lanes) */
   int n_emitters;
   int palette_in_shared;  /* palette size if staged in shared memory, else 0 */
   int spectrum_in_shared; /* 1 when ne <= kSpectrumSharedMax */
@@ -104,6 +105,7 @@ struct TransportParams {
   int max_rejections;     /* iterations per sampler rejection loop before the guard drops the photon */
   float prompt_energy;    /* prompt gamma per decay (eV), 0 = none */
   float prompt_yield;     /* its probability per decay (1: no draw) */
+  int spread_lanes;       /* 1: the longest lanes start on warps of their own */
 };
 
 /* Device pointers of one scene (all read-only during transport). */
@@ -132,7 +134,7 @@ struct DeviceTallies {
   unsigned long long* coincidences;
   unsigned long long* counters;   /* 10 counters (mcpet_counters order) or NULL */
   unsigned long long* guard;      /* guard trips */
-  unsigned long long* lane_cursor;/* lane work queue head */
+  unsigned long long* lane_cursor;/* lane work queue head, zero at the launch */
   const unsigned long long* plan_counts; /* [lanes, emitters] on the device (device-built plans) */
   unsigned long long* mat_dose;   /* [15][2] material dose tally, or NULL */
   unsigned long long* vox_dose;    /* [ROI voxels][2] voxel dose tally, or NULL */

@@ -79,6 +79,21 @@ __device__ __forceinline__ uint64_t claim_lane(unsigned long long* cursor) {
   return base + __popc(mask & ((1u << lane_id) - 1u));
 }
 
+/* The lanes a grid starts with when they are spread (TransportParams::
+ * spread_lanes): the lane of rank r -- plans are ordered by decreasing work --
+ * goes to warp r mod W of the grid's W warps, warps counted across the blocks
+ * first, so that the longest lanes start on warps of their own on different
+ * SMs; later ones come from the work queue, after the first gridDim *
+ * blockDim.  A lane is one serial chain of decays, and in a full warp it
+ * waits for the rounds of 31 others: 25.8 us a decay with 32 of the hot
+ * lanes of a 9^3 cube to a warp, 8.3 us with one (1e7 decays, 96 lanes of
+ * 30458 decays each: 787 -> 253 ms).  Elsewhere the queue deals every lane,
+ * in groups of consecutive ones that share voxels and scenes. */
+__device__ __forceinline__ uint64_t initial_lane() {
+  const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+  return (threadIdx.x & 31) * warps + (uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+}
+
 /* The emitter of a lane: the last one whose first lane is not after it.  Eight
  * ways at a time: a plan of 480 000 emitters takes 7 rounds of independent
  * loads instead of 19 loads that wait for one another. */
@@ -436,7 +451,7 @@ __global__ void __launch_bounds__(kBlock) transport_kernel(TransportParams P, De
   const DoseSink dose{O.mat_dose ? mdose_sh : nullptr, O.vox_dose};
   const bool dose_on = O.mat_dose || O.vox_dose;
   for (;;) {
-    uint64_t lane = claim_lane(O.lane_cursor);
+    uint64_t lane = P.first_lane + claim_lane(O.lane_cursor);
     if (lane >= P.n_lanes) break;
     const Emitter* em = T.emitters + find_emitter(T.emitters, P.n_emitters, lane);
     const int voxel = (int)__ldg(&em->voxel);
@@ -666,6 +681,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) transport_events_kernel(Tr
   Rng rng = {0, 0};
   int phase = kPhDecay;
   bool lane_live = false;
+  bool first_claim = P.spread_lanes != 0;
   int which = 1;            /* photon of the pair being tracked */
   bool fresh = false;       /* next step starts a new interaction-loop iteration */
   bool escaped = false;
@@ -913,7 +929,10 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) transport_events_kernel(Tr
       if (phase == kPhDecay) {
         for (;;) {
           if (__builtin_expect(!lane_live, 0)) {   /* rare branches hinted: cold code out of the hot paths */
-            const uint64_t lane = claim_lane(O.lane_cursor);
+            uint64_t lane = P.first_lane;
+            if (__builtin_expect(first_claim, 0)) lane += initial_lane();
+            else lane += claim_lane(O.lane_cursor) + (P.spread_lanes ? gridDim.x * blockDim.x : 0);
+            first_claim = false;
             if (lane >= n_lanes) {
               phase = kPhDone;
               break;
