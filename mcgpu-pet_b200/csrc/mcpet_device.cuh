@@ -342,17 +342,20 @@ __device__ __forceinline__ bool sample_rayleigh(Rng& r, float energy, int mat, f
   double xlast = (double)__ldg(&R.xco[base + kNpRayleigh - 1]);
   double x2max = ((xmax * xmax) < xlast) ? (xmax * xmax) : xlast;
   if (xmax < 0.01) {
+#pragma unroll 1
     for (int it = 0; it < max_rejections; ++it) {
       costh = 1.0 - ranecu_double(r) * 2.0;
       if (!(ranecu_double(r) > ((costh * costh + 1.0) * 0.5))) return true;
     }
     return false;
   }
+#pragma unroll 1
   for (int it = 0; it < max_rejections; ++it) {
     double ru = ranecu_double(r) * (double)pmax;
     int itn = (int)(ru * (kNpRayleigh - 1));
     int lo = (int)__ldg(&R.itl[itn + base]);
     int hi = (int)__ldg(&R.itu[itn + base]);
+#pragma unroll 1
     while ((hi - lo) > 1) {
       int mid = (lo + hi) >> 1;
       if (ru > (double)__ldg(&R.pco[mid - 1 + base])) lo = mid;
@@ -391,6 +394,7 @@ __device__ __forceinline__ bool sample_rayleigh(Rng& r, float energy, int mat, f
 __device__ __forceinline__ float compton_s0(float E, int mat, const ComptonTable& C) {
   const int nsh = C.noscco[mat];
   float s0 = 0.0f;
+#pragma unroll 1
   for (int i = 0; i < nsh; ++i) {
     float u = C.uico[mat + i * kMaxMaterials];
     if (u < E) {
@@ -408,30 +412,37 @@ __device__ __forceinline__ float compton_s0(float E, int mat, const ComptonTable
   return s0;
 }
 
-/* One trial of GCOa's first stage (MCGPU-PET_kernel.cu:1390-1451): tau = E'/E
- * from the Klein-Nishina-like envelope, then the rejection on the incoherent
- * scattering function, normalised by s0 (compton_s0 of E and the material).
- * Returns true on acceptance, with tau, cdt1 = 1 - cos(theta), the sum s and
- * the shell terms rn[] that the second stage reads.  A trial draws the same
- * random numbers whether the trials of one sampling run back to back or
- * with other work of the thread between them.  kFast (balanced lanes): the
- * envelope branch and cdt1 in single precision instead of the reference's
- * double-precision constant and division. */
-template <bool kFast = false, typename Scratch>
-__device__ __forceinline__ bool compton_trial(Rng& r, float E, int mat, const ComptonTable& C, Scratch rn,
-                                              float s0, float& tau, float& s, double& cdt1) {
-  const int nsh = C.noscco[mat];
+/* A trial of GCOa's first stage (MCGPU-PET_kernel.cu:1390-1451) in two
+ * parts.  The envelope part makes the trial's three draws and gives tau = E'/E
+ * from the Klein-Nishina-like envelope, cdt1 = 1 - cos(theta) and the draw u of
+ * the rejection test; it returns false when the test fails whatever the sum
+ * over the shells: the sum is at most the normaliser s0 (it grows with theta,
+ * and s0 is its value at pi or a bound of that), so a draw above the
+ * Klein-Nishina factor, by a margin far over the rounding of both sums, is
+ * rejected.  The shell part evaluates the sum and the test itself for the
+ * draws that are left.  At 511 keV the first rejects 4 in 10 trials and the
+ * second 1 in 50, so that callers repeat the cheap part until (nearly) all
+ * their lanes have a candidate and evaluate the shells -- a square root and an
+ * exponential each -- once a sampling, with full warps.  A trial draws the
+ * same random numbers whatever part ends it, and whether the trials of one
+ * sampling run back to back or with other work of the thread between them.
+ * kFast (balanced lanes): the envelope branch and cdt1 in single precision
+ * instead of the reference's double-precision constant and division. */
+template <bool kFast = false>
+__device__ __forceinline__ bool compton_envelope(Rng& r, float E, float& tau, double& cdt1, float& u) {
   float ek = E * 1.956951306108245e-6f;
   float ek2 = ek * 2.f + 1.f;
   float ek3 = ek * ek;
   float taumin = 1.f / ek2;
   float a1 = logf(ek2);
-  const bool first_branch = kFast ? (ranecu(r) * (a1 + 2.f * ek * (ek + 1.f) * taumin * taumin) < a1)
+  const bool first_branch = kFast ? (ranecu(r) * __fmaf_rn(2.f * ek * (ek + 1.f) * taumin, taumin, a1) < a1)
                                    : (ranecu(r) * (a1 + 2. * ek * (ek + 1.f) * taumin * taumin) < a1);
+  const float r2 = ranecu(r);
+  u = ranecu(r);
   if (first_branch) {
-    tau = powf(taumin, ranecu(r));
+    tau = powf(taumin, r2);
   } else {
-    tau = sqrtf(1.f + ranecu(r) * (taumin * taumin - 1.f));
+    tau = sqrtf(__fmaf_rn(r2, __fmaf_rn(taumin, taumin, -1.f), 1.f));
   }
   if (kFast) {
     float c = (1.f - tau) / (tau * ek);
@@ -441,31 +452,47 @@ __device__ __forceinline__ bool compton_trial(Rng& r, float E, int mat, const Co
     cdt1 = (double)(1.f - tau) / (((double)tau) * ((double)E) * 1.956951306108245e-6);
     if (cdt1 > 2.0) cdt1 = 1.99999999;
   }
+  return !(u * (ek3 * tau * (tau * tau + 1.0f)) >
+           1.001f * (1.0f + tau * ((ek3 - ek2 - 1.0f) + tau * (ek2 + tau * ek3))));
+}
+
+/* The shell part: the incoherent scattering function s at the candidate's
+ * angle, its shell terms rn[] that the second stage reads, and the rejection
+ * test normalised by s0 (compton_s0 of E and the material, or a bound).  Which
+ * products round before their sum is spelled out: left to the compiler it
+ * differed between the kernel's variants, and a history in 1e9 with it. */
+template <typename Scratch>
+__device__ __forceinline__ bool compton_shells(float E, int mat, const ComptonTable& C, Scratch rn, float s0,
+                                               float tau, double cdt1, float u_test, float& s) {
+  const int nsh = C.noscco[mat];
+  float ek = E * 1.956951306108245e-6f;
+  float ek2 = ek * 2.f + 1.f;
+  const float ek3 = __fmul_rn(ek, ek);
   s = 0.0f;
+#pragma unroll 1
   for (int i = 0; i < nsh; ++i) {
     float u = C.uico[mat + i * kMaxMaterials];
     if (u < E) {
       float aux = E * (E - u) * ((float)cdt1);
       float pz;
       if ((aux > 1.0e-12f) || (u > 1.0e-12f)) {
-        pz = C.fj0[mat + i * kMaxMaterials] * (aux - u * 510998.918f) * rsqrtf(aux + aux + u * u) *
+        pz = C.fj0[mat + i * kMaxMaterials] * __fmaf_rn(-u, 510998.918f, aux) * rsqrtf(__fmaf_rn(u, u, aux + aux)) *
              1.956951306108245e-6f;
       } else {
         pz = 0.002f;
       }
-      float t = pz * 1.4142135623731f;
-      if (pz > 0.0f) t = 0.5f - (t + 0.70710678118654502f) * (t + 0.70710678118654502f);
-      else t = 0.5f - (0.70710678118654502f - t) * (0.70710678118654502f - t);
-      t = 0.5f * expf(t);
+      const float w = __fmaf_rn(fabsf(pz), 1.4142135623731f, 0.70710678118654502f);
+      float t = 0.5f * expf(__fsub_rn(0.5f, __fmul_rn(w, w)));
       if (pz > 0.0f) t = 1.0f - t;
-      s += C.fco[mat + i * kMaxMaterials] * t;
+      s = __fmaf_rn(C.fco[mat + i * kMaxMaterials], t, s);
       rn[i] = t;
     } else {
       rn[i] = 0.0f;   /* shell above the photon energy: the reference leaves it uninitialised */
     }
   }
-  return !((ranecu(r) * s0) >
-           (s * (1.0f + tau * ((ek3 - ek2 - 1.0f) + tau * (ek2 + tau * ek3)))) / (ek3 * tau * (tau * tau + 1.0f)));
+  const float k = __fadd_rn(ek2, __fmul_rn(tau, ek3));
+  const float f = __fmaf_rn(tau, __fmaf_rn(tau, k, __fsub_rn(__fsub_rn(ek3, ek2), 1.0f)), 1.0f);
+  return !(u_test * s0 > s * f / (ek3 * tau * __fmaf_rn(tau, tau, 1.0f)));
 }
 
 /* GCOa's second stage after an accepted trial (MCGPU-PET_kernel.cu:1453-1562):
@@ -485,6 +512,7 @@ __device__ __forceinline__ bool compton_doppler(Rng& r, float& energy, int mat, 
     float t = s * ranecu(r);
     float pac = 0.0f;
     int ish = nsh - 1;
+#pragma unroll 1
     for (int i = 0; i < (nsh - 1); ++i) {
       pac += C.fco[mat + i * kMaxMaterials] * rn[i];
       if (pac > t) {
@@ -537,13 +565,14 @@ __device__ __forceinline__ bool sample_compton(Rng& r, float& energy, int mat, c
                                                int max_rejections = kMaxRejections) {
   const float E = energy;
   const float s0 = s0_given < 0.0f ? compton_s0(E, mat, C) : s0_given;
-  float tau, s;
+  float tau, s, u;
   double cdt1;
   int it = 0;
-  for (;;) {
-    if (++it > max_rejections) return false;
-    if (compton_trial<kFast>(r, E, mat, C, rn, s0, tau, s, cdt1)) break;
-  }
+  do {
+    do {
+      if (++it > max_rejections) return false;
+    } while (!compton_envelope<kFast>(r, E, tau, cdt1, u));
+  } while (!compton_shells(E, mat, C, rn, s0, tau, cdt1, u, s));
   costh = 1.0 - cdt1;
   return compton_doppler<kFast>(r, energy, mat, C, rn, tau, s, costh, max_rejections);
 }

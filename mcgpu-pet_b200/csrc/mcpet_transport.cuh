@@ -761,8 +761,10 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) transport_events_kernel(Tr
        * Rayleigh (:375-387), then the common direction update.  Rayleigh
        * lanes (GRAa) join a round with Compton lanes only when at least
        * quorum_rayleigh of them wait, so that most rounds run one sampler.
-       * The Compton lanes repeat trials of GCOa's first stage until at most
-       * an eighth of them are still rejected; those keep their phase and go
+       * The Compton lanes repeat the envelope part of GCOa's first stage
+       * until at most an eighth of them lacks a candidate, then evaluate the
+       * shells of all candidates at once, and so on until at most an eighth
+       * is still rejected; those keep their phase and go
        * on in a later round, with the lanes that arrive meanwhile, instead of
        * holding the warp in the rejection loop (each lane draws its random
        * numbers in the same order either way) */
@@ -787,13 +789,20 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) transport_events_kernel(Tr
           } else {
             s0 = cold.f(kCS0);
           }
-          float tau = 0.f, s = 0.f;
+          float tau = 0.f, s = 0.f, u = 0.f;
           double cdt1 = 0.0;
-          bool accepted = false, tripped = false;
+          bool accepted = false, tripped = false, candidate = false;
           for (;;) {
-            if (!accepted && !tripped) {
-              if (++trials > (uint32_t)rejections_cap<kMode>(P)) tripped = true;
-              else accepted = compton_trial<(kMode & kModeFast) != 0>(rng, e, mat0, cmp, rn, s0, tau, s, cdt1);
+            for (;;) {
+              if (!accepted && !tripped && !candidate) {
+                if (++trials > (uint32_t)rejections_cap<kMode>(P)) tripped = true;
+                else candidate = compton_envelope<(kMode & kModeFast) != 0>(rng, e, tau, cdt1, u);
+              }
+              if (8 * __popc(__ballot_sync(m_c, !accepted && !tripped && !candidate)) <= __popc(m_c)) break;
+            }
+            if (candidate) {
+              accepted = compton_shells(e, mat0, cmp, rn, s0, tau, cdt1, u, s);
+              candidate = false;
             }
             if (8 * __popc(__ballot_sync(m_c, !accepted && !tripped)) <= __popc(m_c)) break;
           }
