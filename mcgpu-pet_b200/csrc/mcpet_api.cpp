@@ -64,14 +64,6 @@ int env_int(const char* name, int def, int lo, int hi) {
   return x < lo ? lo : (x > hi ? hi : x);
 }
 
-Divisor divisor(int d) {
-  Divisor r = {0, 0};
-  if (d < 1) return r;
-  while ((1ll << r.s) < d) ++r.s;
-  r.m = (uint32_t)(((1ull << (31 + r.s)) + (uint32_t)d - 1) / (uint32_t)d);
-  return r;
-}
-
 void fill_params(const mcpet_scene* sc, TransportParams& P) {
   memset(&P, 0, sizeof(P));
   const mcpet_config& c = sc->cfg;
@@ -112,9 +104,6 @@ void fill_params(const mcpet_scene* sc, TransportParams& P) {
   P.span = c.span;
   P.nsinos = c.n_sinograms;
   P.nbins = c.n_bins;
-  P.div_nx = divisor(P.nx);
-  P.div_ny = divisor(P.ny);
-  P.div_ncrystals = divisor(P.ncrystals);
   P.seed = c.seed;
   int ms = 1;
   for (int m = 0; m < kMaxMaterials; ++m)

@@ -130,10 +130,6 @@ __device__ __forceinline__ Rng rng_stream(int seed, uint64_t stream) {
   return r;
 }
 
-__device__ __forceinline__ uint32_t divide(uint32_t v, const Divisor& d) {
-  return (uint32_t)(((uint64_t)v * d.m) >> (31 + d.s));
-}
-
 /* ------------------------------------------------------------------------
  * Voxel lookup (locate_voxel, MCGPU-PET_kernel.cu:1098-1124). */
 __device__ __forceinline__ int locate(const TransportParams& P, float x, float y, float z) {
@@ -659,29 +655,27 @@ __device__ __forceinline__ long long sinogram_bin(const TransportParams& P, floa
   int iseg = 2 * incl;
   if (zb < za && iseg > 0) iseg -= 1;
   /* first plane of segment iseg: iseg*NZS minus the planes the oblique
-   * segments lack (closed form of the reference's running sum; below twice
-   * the number of planes, an int) */
-  int ofseg = iseg * P.nzs;
+   * segments lack (closed form of the reference's running sum) */
+  long long ofseg = (long long)iseg * P.nzs;
   if (iseg >= 2) {
-    const int n = iseg - 2;
-    ofseg -= (iseg - 1) * (P.span + 1);
-    ofseg -= 2 * P.span * ((n / 2) * ((n + 1) / 2));
+    long long n = iseg - 2;
+    ofseg -= (long long)(iseg - 1) * (P.span + 1);
+    ofseg -= 2LL * P.span * ((n / 2) * ((n + 1) / 2));
   }
   int ofz = 0;
   if (incl > 0) ofz = ((P.span + 1) / 2) + (incl - 1) * P.span;
-  const int izm = ofseg + (za + zb) - ofz;
+  long long izm = ofseg + (za + zb) - ofz;
   if (xb < xa) {
     int t = xa;
     xa = xb;
     xb = t;
   }
-  const uint32_t turn = (uint32_t)(xa + xb + P.nangles + 1);
-  int ith = (int)(turn - divide(turn, P.div_ncrystals) * (uint32_t)P.ncrystals) / 2;
+  int ith = ((xa + xb + P.nangles + 1) % P.ncrystals) / 2;
   int ir = abs(xb - xa - P.nangles);
   if ((xa < ith) || (xb >= (ith + P.nangles))) ir = -ir;
   ir = ir + P.nrad / 2;
   if (izm < 0 || izm >= P.nsinos || ir < 0 || ir >= P.nrad) return -1;
-  return ((long long)izm * P.nangles + ith) * P.nrad + ir;
+  return izm * (long long)P.nangles * P.nrad + (long long)ith * P.nrad + ir;
 }
 
 /* Gaussian energy blur of one photon as drawn by the sinogram tally

@@ -13,13 +13,6 @@ constexpr int kLeapHistories = 555555;  /* histories_per_thread of the jump, MCG
 constexpr int kLeapDistance = 256;      /* LEAP_DISTANCE, MCGPU-PET_kernel.cu:898 */
 constexpr int kSpectrumSharedMax = 4096; /* spectrum bins privatised in shared memory */
 
-/* Division by a launch constant d >= 1 as a product: (v m) >> (31 + s) with
- * 2^s >= d and m = ceil(2^(31+s) / d) is v / d for every v < 2^31 (v times the
- * excess of m d over 2^(31+s), which is below d <= 2^s, stays below 2^(31+s)). */
-struct Divisor {
-  uint32_t m, s;
-};
-
 /* Interaction record for one (energy bin, material): the interpolation
  * coefficients of the three inverse mean free paths (total, Compton,
  * Rayleigh; reference mfp_table_a/b, MCGPU-PET.cu:1688-1746) interleaved with
@@ -112,7 +105,6 @@ struct TransportParams {
   int max_rejections;     /* iterations per sampler rejection loop before the guard drops the photon */
   float prompt_energy;    /* prompt gamma per decay (eV), 0 = none */
   float prompt_yield;     /* its probability per decay (1: no draw) */
-  Divisor div_nx, div_ny, div_ncrystals;
   int spread_lanes;       /* 1: the longest lanes start on warps of their own */
 };
 

@@ -1125,8 +1125,7 @@ __global__ void __launch_bounds__(kBlock, kCount ? kMinBlocks : resident_blocks(
             cold.u(F.rx) = (uint32_t)rng.x;
             cold.u(F.rx + 1) = (uint32_t)rng.y;
           }
-          const int row = (int)divide((uint32_t)voxel, PN.div_nx), plane = (int)divide((uint32_t)row, PN.div_ny);
-          emit_first(rng, PN, voxel - row * PN.nx, row - plane * PN.ny, plane, ph.pos, ph.dir);
+          emit_first(rng, PN, voxel % PN.nx, (voxel / PN.nx) % PN.ny, voxel / (PN.nx * PN.ny), ph.pos, ph.dir);
           cold.set_vec(F.o, ph.pos);
           cold.set_vec(F.d, ph.dir);
           which = 1;
