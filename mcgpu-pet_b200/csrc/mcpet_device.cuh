@@ -387,47 +387,26 @@ __device__ __forceinline__ bool sample_rayleigh(Rng& r, float energy, int mat, f
  * MCGPU-PET_kernel.cu:1335-1563).  `C` is the block's shared copy of the
  * shell table, `rn` a per-thread scratch of max_shells floats.  Updates the
  * energy; returns false when a rejection guard fired. */
-/* A block's copy of the shell table in shared memory: {uico, fj0, fco} of a
- * shell in one 16-byte word, [shell][material], only as many shells as the
- * launch's materials have (9 of 30 for air and water: 2.2 KB instead of 5.5,
- * which the fourth resident block of the event kernel needs), and one load a
- * shell instead of three. */
-struct ShellTable {
-  const float4* row;
-  const int* noscco;
-};
-__host__ __device__ constexpr int shell_table_bytes(int shells) { return shells * kMaxMaterials * 16 + 64; }
-__device__ __forceinline__ ShellTable stage_shells(char*& at, const ComptonTable* src, int shells) {
-  float4* row = reinterpret_cast<float4*>(at);
-  int* n = reinterpret_cast<int*>(row + shells * kMaxMaterials);
-  at += shell_table_bytes(shells);
-  for (int i = threadIdx.x; i < shells * kMaxMaterials; i += blockDim.x)
-    row[i] = make_float4(__ldg(&src->uico[i]), __ldg(&src->fj0[i]), __ldg(&src->fco[i]), 0.0f);
-  for (int i = threadIdx.x; i < kMaxMaterials; i += blockDim.x) n[i] = __ldg(&src->noscco[i]);
-  return ShellTable{row, n};
-}
-
 /* Incoherent scattering function at theta = pi, the normalisation of the
  * rejection step of GCOa (MCGPU-PET_kernel.cu:1366-1391).  It depends only on
  * the energy and material, so kernels evaluate it once per block for the
  * annihilation energy and pass the value in. */
-__device__ __forceinline__ float compton_s0(float E, int mat, const ShellTable& C) {
+__device__ __forceinline__ float compton_s0(float E, int mat, const ComptonTable& C) {
   const int nsh = C.noscco[mat];
   float s0 = 0.0f;
 #pragma unroll 1
   for (int i = 0; i < nsh; ++i) {
-    const float4 sh = C.row[mat + i * kMaxMaterials];
-    float u = sh.x;
+    float u = C.uico[mat + i * kMaxMaterials];
     if (u < E) {
       float aux = E * (E - u) * 2.f;
-      float pz = sh.y * (aux - u * 510998.918f) *
+      float pz = C.fj0[mat + i * kMaxMaterials] * (aux - u * 510998.918f) *
                  rsqrtf(aux + aux + u * u) * 1.956951306108245e-6f;
       float t;
       if (pz > 0.0f) t = (0.707106781186545f + pz * 1.4142135623731f) * (0.707106781186545f + pz * 1.4142135623731f);
       else t = (0.707106781186545f - pz * 1.4142135623731f) * (0.707106781186545f - pz * 1.4142135623731f);
       t = 0.5f * expf(0.5f - t);
       if (pz > 0.0f) t = 1.0f - t;
-      s0 += sh.z * t;
+      s0 += C.fco[mat + i * kMaxMaterials] * t;
     }
   }
   return s0;
@@ -484,7 +463,7 @@ __device__ __forceinline__ bool compton_envelope(Rng& r, float E, float& tau, do
  * products round before their sum is spelled out: left to the compiler it
  * differed between the kernel's variants, and a history in 1e9 with it. */
 template <typename Scratch>
-__device__ __forceinline__ bool compton_shells(float E, int mat, const ShellTable& C, Scratch rn, float s0,
+__device__ __forceinline__ bool compton_shells(float E, int mat, const ComptonTable& C, Scratch rn, float s0,
                                                float tau, double cdt1, float u_test, float& s) {
   const int nsh = C.noscco[mat];
   float ek = E * 1.956951306108245e-6f;
@@ -493,13 +472,12 @@ __device__ __forceinline__ bool compton_shells(float E, int mat, const ShellTabl
   s = 0.0f;
 #pragma unroll 1
   for (int i = 0; i < nsh; ++i) {
-    const float4 sh = C.row[mat + i * kMaxMaterials];
-    float u = sh.x;
+    float u = C.uico[mat + i * kMaxMaterials];
     if (u < E) {
       float aux = E * (E - u) * ((float)cdt1);
       float pz;
       if ((aux > 1.0e-12f) || (u > 1.0e-12f)) {
-        pz = sh.y * __fmaf_rn(-u, 510998.918f, aux) * rsqrtf(__fmaf_rn(u, u, aux + aux)) *
+        pz = C.fj0[mat + i * kMaxMaterials] * __fmaf_rn(-u, 510998.918f, aux) * rsqrtf(__fmaf_rn(u, u, aux + aux)) *
              1.956951306108245e-6f;
       } else {
         pz = 0.002f;
@@ -507,7 +485,7 @@ __device__ __forceinline__ bool compton_shells(float E, int mat, const ShellTabl
       const float w = __fmaf_rn(fabsf(pz), 1.4142135623731f, 0.70710678118654502f);
       float t = 0.5f * expf(__fsub_rn(0.5f, __fmul_rn(w, w)));
       if (pz > 0.0f) t = 1.0f - t;
-      s = __fmaf_rn(sh.z, t, s);
+      s = __fmaf_rn(C.fco[mat + i * kMaxMaterials], t, s);
       rn[i] = t;
     } else {
       rn[i] = 0.0f;   /* shell above the photon energy: the reference leaves it uninitialised */
@@ -524,7 +502,7 @@ __device__ __forceinline__ bool compton_shells(float E, int mat, const ShellTabl
  * Returns false when the rejection guard fired.  kFast (balanced lanes):
  * the angle term in single precision (the reference's mixes in double). */
 template <bool kFast = false, typename Scratch>
-__device__ __forceinline__ bool compton_doppler(Rng& r, float& energy, int mat, const ShellTable& C, Scratch rn,
+__device__ __forceinline__ bool compton_doppler(Rng& r, float& energy, int mat, const ComptonTable& C, Scratch rn,
                                                 float tau, float s, double costh,
                                                 int max_rejections = kMaxRejections) {
   const int nsh = C.noscco[mat];
@@ -537,7 +515,7 @@ __device__ __forceinline__ bool compton_doppler(Rng& r, float& energy, int mat, 
     int ish = nsh - 1;
 #pragma unroll 1
     for (int i = 0; i < (nsh - 1); ++i) {
-      pac += C.row[mat + i * kMaxMaterials].z * rn[i];
+      pac += C.fco[mat + i * kMaxMaterials] * rn[i];
       if (pac > t) {
         ish = i;
         break;
@@ -546,10 +524,10 @@ __device__ __forceinline__ bool compton_doppler(Rng& r, float& energy, int mat, 
     t = ranecu(r) * rn[ish];
     if (t < 0.5f) {
       pzomc = (0.70710678118654502f - sqrtf(0.5f - logf(t + t))) /
-              (C.row[mat + ish * kMaxMaterials].y * 1.4142135623731f);
+              (C.fj0[mat + ish * kMaxMaterials] * 1.4142135623731f);
     } else {
       pzomc = (sqrtf(0.5f - logf(2.0f - 2.0f * t)) - 0.70710678118654502f) /
-              (C.row[mat + ish * kMaxMaterials].y * 1.4142135623731f);
+              (C.fj0[mat + ish * kMaxMaterials] * 1.4142135623731f);
     }
     if (pzomc < -1.0f) continue;
     t = kFast ? tau * (tau - (float)costh * 2.f) + 1.f : tau * (tau - costh * 2.f) + 1.f;
@@ -583,7 +561,7 @@ __device__ __forceinline__ bool compton_doppler(Rng& r, float& energy, int mat, 
  * s0 < 0: the normaliser evaluated at the photon's energy (the reference's
  * arithmetic); else the bound given (MfpRecord::s0_bound). */
 template <bool kFast = false, typename Scratch>
-__device__ __forceinline__ bool sample_compton(Rng& r, float& energy, int mat, const ShellTable& C,
+__device__ __forceinline__ bool sample_compton(Rng& r, float& energy, int mat, const ComptonTable& C,
                                                Scratch rn, double& costh, float s0_given = -1.0f,
                                                int max_rejections = kMaxRejections) {
   const float E = energy;

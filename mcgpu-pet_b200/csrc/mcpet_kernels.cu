@@ -82,13 +82,17 @@ __global__ void probe_detector_kernel(TransportParams P, DeviceTallies O, int n,
 
 __global__ void probe_compton_kernel(const ComptonTable* tab, int n, float* energy, const int* mat, int2* seeds,
                                      double* costh, int max_shells) {
+  __shared__ ComptonTable cmp;
   extern __shared__ float4 dyn_smem[];
-  char* cursor = reinterpret_cast<char*>(dyn_smem);
-  const ShellTable cmp = stage_shells(cursor, tab, max_shells);
+  {
+    const int* src = reinterpret_cast<const int*>(tab);
+    int* dst = reinterpret_cast<int*>(&cmp);
+    for (int i = threadIdx.x; i < (int)(sizeof(ComptonTable) / 4); i += blockDim.x) dst[i] = src[i];
+  }
   __syncthreads();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  SharedScratch rn{reinterpret_cast<float*>(cursor) + threadIdx.x, (int)blockDim.x};
+  SharedScratch rn{reinterpret_cast<float*>(dyn_smem) + threadIdx.x, (int)blockDim.x};
   Rng r;
   r.x = seeds[i].x;
   r.y = seeds[i].y;
@@ -178,11 +182,16 @@ __global__ void __launch_bounds__(kBlock) grad_replay_kernel(TransportParams P, 
                                                              const int* trues, const int* scatter, const float* bg,
                                                              const float* activity, float* grad_a, float* grad_s,
                                                              unsigned long long* stats) {
+  __shared__ ComptonTable cmp;
   extern __shared__ float4 dyn_smem[];
-  char* cursor = reinterpret_cast<char*>(dyn_smem);
-  const ShellTable cmp = stage_shells(cursor, T.compton, P.max_shells > 0 ? P.max_shells : 1);
+  float* scratch = reinterpret_cast<float*>(dyn_smem);
+  {
+    const int* src = reinterpret_cast<const int*>(T.compton);
+    int* dst = reinterpret_cast<int*>(&cmp);
+    for (int i = threadIdx.x; i < (int)(sizeof(ComptonTable) / 4); i += blockDim.x) dst[i] = __ldg(&src[i]);
+  }
   __syncthreads();
-  SharedScratch rn{reinterpret_cast<float*>(cursor) + threadIdx.x, (int)blockDim.x};
+  SharedScratch rn{scratch + threadIdx.x, (int)blockDim.x};
   const bool background = P.background_mode != 0;
   unsigned long long ok_count = 0, bad_count = 0;
   LaneCounters cnt = {};
@@ -502,8 +511,7 @@ static size_t dynamic_smem(const TransportParams& P, int block, int algorithm, i
   size_t s = 0;
   if (P.spectrum_in_shared) s += ((size_t)P.ne * 4 + 15) / 16 * 16;
   if (P.palette_in_shared) s += ((size_t)P.palette_in_shared * sizeof(PaletteEntry) + 15) / 16 * 16;
-  const int shells = P.max_shells > 0 ? P.max_shells : 1;
-  s += (size_t)shell_table_bytes(shells) + (size_t)shells * block * sizeof(float);
+  s += (size_t)(P.max_shells > 0 ? P.max_shells : 1) * block * sizeof(float);
   if (algorithm != kAlgorithmHistories)
     s += (size_t)lane_words(mode, batch, algorithm == kAlgorithmEventsRecord) * block * sizeof(uint32_t);
   return s;
@@ -606,8 +614,7 @@ cudaError_t launch_grad_replay(const TransportParams& P, const DeviceTables& T, 
                                unsigned long long* stats, int sm_count, int mode, cudaStream_t stream) {
   /* the replay recomputes histories with the forward run's arithmetic */
   auto kernel = (mode & kModeFast) ? grad_replay_kernel<kModeFast> : grad_replay_kernel<0>;
-  const int shells = P.max_shells > 0 ? P.max_shells : 1;
-  const size_t smem = (size_t)shell_table_bytes(shells) + (size_t)shells * kBlock * sizeof(float);
+  const size_t smem = (size_t)(P.max_shells > 0 ? P.max_shells : 1) * kBlock * sizeof(float);
   cudaError_t e = occupancy_smem_attr(kernel, smem);
   if (e != cudaSuccess) return e;
   int bps = 0;
@@ -645,7 +652,7 @@ cudaError_t launch_probe_detector(const TransportParams& P, int n, const float* 
 
 cudaError_t launch_probe_compton(const ComptonTable* tab, int n, float* energy, const int* mat, int2* seeds,
                                  double* costh, cudaStream_t s) {
-  size_t smem = (size_t)shell_table_bytes(kMaxShells) + (size_t)kMaxShells * 128 * sizeof(float);
+  size_t smem = (size_t)kMaxShells * 128 * sizeof(float);
   probe_compton_kernel<<<(n + 127) / 128, 128, smem, s>>>(tab, n, energy, mat, seeds, costh, kMaxShells);
   return cudaGetLastError();
 }

@@ -165,7 +165,7 @@ struct NoStepHook {
  * interaction selection of MCGPU-PET_kernel.cu:298-414. */
 template <bool kCount, int kMode, typename Scratch, typename Hook = NoStepHook>
 __device__ __forceinline__ bool track_photon(Rng& rng, const TransportParams& P, const DeviceTables& T,
-                                             const PaletteEntry* pal, const ShellTable& C, Scratch rn,
+                                             const PaletteEntry* pal, const ComptonTable& C, Scratch rn,
                                              PhotonState& ph, LaneCounters& cnt, Hook* hook = nullptr,
                                              const DoseSink* dose = nullptr) {
   float energy = ph.energy;
@@ -414,10 +414,11 @@ constexpr int kBlock = 256;
 template <bool kCount, int kMode>
 __global__ void __launch_bounds__(kBlock) transport_kernel(TransportParams P, DeviceTables T, DeviceTallies O) {
   constexpr bool kFastLanes = (kMode & kModeFast) != 0;
+  __shared__ ComptonTable cmp;
   __shared__ unsigned long long mdose_sh[2 * kMaxMaterials];
   if (threadIdx.x < 2 * kMaxMaterials) mdose_sh[threadIdx.x] = 0;
   extern __shared__ float4 dyn_smem[];
-  /* dynamic shared layout: [spectrum ints][palette entries][shell table][rn scratch] */
+  /* dynamic shared layout: [spectrum ints][palette entries][rn scratch] */
   int* spec_sh = nullptr;
   char* cursor = reinterpret_cast<char*>(dyn_smem);
   if (P.spectrum_in_shared) {
@@ -431,10 +432,12 @@ __global__ void __launch_bounds__(kBlock) transport_kernel(TransportParams P, De
     cursor += ((P.palette_in_shared * (int)sizeof(PaletteEntry) + 15) / 16) * 16;
     pal = pal_sh;
   }
-  const ShellTable cmp = stage_shells(cursor, T.compton, P.max_shells > 0 ? P.max_shells : 1);
   SharedScratch rn{reinterpret_cast<float*>(cursor) + threadIdx.x, (int)blockDim.x};
 
   {
+    const int* src = reinterpret_cast<const int*>(T.compton);
+    int* dst = reinterpret_cast<int*>(&cmp);
+    for (int i = threadIdx.x; i < (int)(sizeof(ComptonTable) / 4); i += blockDim.x) dst[i] = __ldg(&src[i]);
     if (spec_sh)
       for (int i = threadIdx.x; i < P.ne; i += blockDim.x) spec_sh[i] = 0;
     if (pal_sh)
@@ -572,11 +575,7 @@ constexpr float kAbsorbed = -10.0f;
  * that is in the chosen phase (no photon ever leaves its thread): three wide
  * loads and stores and some forty instructions, against the hundreds of the
  * round.  5e7 decays of the head: 17.9e9 instructions of 10.8 threads become
- * 16.2e9 of 13.5; 1e9 decays 354 -> 328 ms with three resident blocks, 300 with
- * four (ShellTable); reference lanes, whose rounds are longer, 87 -> 60 ms at
- * 1e8.  Tried beside it: a phase of its own for the pairs that meet the
- * detector (327 against 300: its lanes wait), no exchange for fewer than four
- * gaining threads (306).  Prompt-gamma variants
+ * 16.3e9 of 13.7; 1e9 decays 354 -> 328 ms.  Prompt-gamma variants
  * keep one lane a thread: their third photon needs the shared memory of two
  * thirds of a lane more, and only two blocks would be resident; and so do the
  * variants for measurements and tests, counters and lowered caps. */
@@ -616,7 +615,7 @@ __host__ __device__ constexpr LaneFields lane_fields(int mode, bool batch, bool 
   f.saved = 12 + (travel ? 1 : 0) + (batch ? 1 : 0);
   return f;
 }
-__host__ __device__ constexpr int lane_words(int mode, bool batch, bool record) {
+constexpr int lane_words(int mode, bool batch, bool record) {
   return lane_fields(mode, batch, record).words * (dual_lanes(mode) ? 2 : 1) +
          (dual_lanes(mode) ? lane_fields(mode, batch, record).saved : 0);
 }
@@ -682,15 +681,14 @@ struct WaitingState {
 constexpr int kShareScanner = kBatchShareScanner;
 constexpr int kSharePhantom = kBatchSharePhantom;
 
-/* Resident blocks that the event kernel's registers are capped for: as many as
- * the shared memory has room for with air's 9 shells. */
-constexpr int resident_blocks(int min_blocks, int mode, bool batch, bool record) {
-  return min_blocks > 3 && lane_words(mode, batch, record) > 40 ? 3 : min_blocks;
-}
+/* Resident blocks that the event kernel's registers are capped for: two lanes
+ * a thread have the shared memory for 3 blocks of 256 (84 registers, no
+ * spills), one lane has it for kMinBlocks. */
+constexpr int resident_blocks(int min_blocks, int mode) { return dual_lanes(mode) && min_blocks > 3 ? 3 : min_blocks; }
 
 template <bool kCount, int kMinBlocks = 1, bool kDevicePlan = false, bool kBatch = false, bool kRecord = false,
           bool kDose = false, int kShare = 0, int kMode = 0>
-__global__ void __launch_bounds__(kBlock, kCount ? kMinBlocks : resident_blocks(kMinBlocks, kMode, kBatch, kRecord)) transport_events_kernel(TransportParams P, DeviceTables T,
+__global__ void __launch_bounds__(kBlock, kCount ? kMinBlocks : resident_blocks(kMinBlocks, kMode)) transport_events_kernel(TransportParams P, DeviceTables T,
                                                                               DeviceTallies O,
                                                                               const SceneSlot* __restrict__ slots,
                                                                               int n_slots) {
@@ -712,6 +710,7 @@ __global__ void __launch_bounds__(kBlock, kCount ? kMinBlocks : resident_blocks(
   const uint64_t n_lanes = kDevicePlan ? (uint64_t)O.plan_counts[0] : P.n_lanes;
   const int n_emitters = kDevicePlan ? (int)O.plan_counts[1] : P.n_emitters;
   __shared__ unsigned long long mdose_sh[2 * kMaxMaterials];
+  __shared__ ComptonTable cmp;
   __shared__ float s0_ann[kMaxMaterials];
   extern __shared__ float4 dyn_smem[];
   int* spec_sh = nullptr;
@@ -727,7 +726,6 @@ __global__ void __launch_bounds__(kBlock, kCount ? kMinBlocks : resident_blocks(
     cursor += ((P.palette_in_shared * (int)sizeof(PaletteEntry) + 15) / 16) * 16;
     pal = pal_sh;
   }
-  const ShellTable cmp = stage_shells(cursor, T.compton, P.max_shells > 0 ? P.max_shells : 1);
   SharedScratch rn{reinterpret_cast<float*>(cursor) + threadIdx.x, (int)blockDim.x};
   cursor += (size_t)(P.max_shells > 0 ? P.max_shells : 1) * blockDim.x * sizeof(float);
   constexpr LaneFields F = lane_fields(kMode, kBatch, kRecord);
@@ -737,6 +735,9 @@ __global__ void __launch_bounds__(kBlock, kCount ? kMinBlocks : resident_blocks(
   if (kDual) cursor += (size_t)F.saved * blockDim.x * sizeof(uint32_t);
   ColdState cold{reinterpret_cast<uint32_t*>(cursor) + threadIdx.x, (int)blockDim.x};   /* of the lane in registers */
   {
+    const int* src = reinterpret_cast<const int*>(T.compton);
+    int* dst = reinterpret_cast<int*>(&cmp);
+    for (int i = threadIdx.x; i < (int)(sizeof(ComptonTable) / 4); i += blockDim.x) dst[i] = __ldg(&src[i]);
     if (spec_sh)
       for (int i = threadIdx.x; i < P.ne; i += blockDim.x) spec_sh[i] = 0;
     if (pal_sh)
