@@ -116,9 +116,7 @@ void fill_params(const mcpet_scene* sc, TransportParams& P) {
       (sc->palette.size() <= 2048 && env_int("MCPET_PALETTE_SHARED", 1, 0, 1)) ? (int)sc->palette.size() : 0;
   P.e_annihilation = 510998.95f;
   for (int k = 0; k < 6; ++k) P.dose_roi[k] = c.tally_voxel_dose ? c.dose_roi[k] : (k % 2 ? -1 : 0);
-  /* with two lanes a thread 20 threads are soon found (1e9-decay head: 16
-   * 310.5 ms, 20 299.8, 24 300.2, 28 312.9); a prompt-gamma scene has one */
-  P.quorum_scatter = env_int("MCPET_QUORUM_SCATTER", c.prompt_gamma_energy > 0.0f ? 16 : 20, 1, 32);
+  P.quorum_scatter = env_int("MCPET_QUORUM_SCATTER", 16, 1, 32);
   P.quorum_pair = env_int("MCPET_QUORUM_PAIR", 16, 1, 32);
   P.step_keep = env_int("MCPET_STEP_KEEP", 2, 1, 8);
   P.quorum_rayleigh = env_int("MCPET_QUORUM_RAYLEIGH", 2, 1, 32);
@@ -592,7 +590,7 @@ mcpet_status launch_planned(mcpet_scene* sc, const mcpet_run_opts& o, TransportP
     if (algorithm != kAlgorithmEvents || (mode & kTransportPrompt)) algorithm = kAlgorithmHistories;
   }
   P.spread_lanes = spread_lanes(d.max_lane_decays, scene_decays(sc));
-  size_t smem = transport_dynamic_smem(P, block, algorithm, mode);
+  size_t smem = transport_dynamic_smem(P, block, algorithm);
   int bps = 0;
   CUDA_TRY(transport_occupancy(counters, algorithm, mode, block, smem, &bps));
   if (bps < 1) return set_error(MCPET_ERR_LIMIT, "transport kernel does not fit on an SM (smem %zu)", smem);
@@ -995,10 +993,8 @@ mcpet_status setup_batch(mcpet_scene* const* scenes, int n, const mcpet_run_opts
     g.P.max_shells = max_shells;
     /* the launch's shared layout holds the prompt-gamma fields when any of
      * its scenes emits one (each lane reads its own scene's emitter) */
-    for (int i = j; i < j + g.count; ++i) {
+    for (int i = j; i < j + g.count; ++i)
       g.P.prompt_energy = std::max(g.P.prompt_energy, L.slots[(size_t)i].P.prompt_energy);
-      g.P.quorum_scatter = std::min(g.P.quorum_scatter, L.slots[(size_t)i].P.quorum_scatter);
-    }
     g.T = L.slots[(size_t)j].T;
     g.T.emitters = nullptr;
     L.groups.push_back(g);
@@ -1026,7 +1022,7 @@ mcpet_status setup_batch(mcpet_scene* const* scenes, int n, const mcpet_run_opts
            (sino_only ? kTransportSinogramOnly : 0);
   for (BatchGroup& g : L.groups) {
     if (g.solo) {
-      g.smem = transport_dynamic_smem(g.P, L.block, g.algorithm, g.mode);
+      g.smem = transport_dynamic_smem(g.P, L.block, g.algorithm);
       int bps = 0;
       CUDA_TRY(transport_occupancy(L.counters, g.algorithm, g.mode, L.block, g.smem, &bps));
       if (bps < 1) return set_error(MCPET_ERR_LIMIT, "transport kernel does not fit on an SM (smem %zu)", g.smem);
@@ -1043,14 +1039,14 @@ mcpet_status setup_batch(mcpet_scene* const* scenes, int n, const mcpet_run_opts
       }
       g.share = (scanner ? kBatchShareScanner : 0) | (phantom ? kBatchSharePhantom : 0);
     }
-    g.smem = transport_batch_dynamic_smem(g.P, L.block, L.mode);
+    g.smem = transport_batch_dynamic_smem(g.P, L.block);
     /* a shared phantom's palette is staged in shared memory, as in a single run */
     if (g.share & kBatchSharePhantom) {
       TransportParams one;
       fill_params(scenes[L.scene_of[(size_t)g.first]], one);
       if (one.palette_in_shared) {
         g.P.palette_in_shared = one.palette_in_shared;
-        g.smem = transport_batch_dynamic_smem(g.P, L.block, L.mode);
+        g.smem = transport_batch_dynamic_smem(g.P, L.block);
       }
     }
     int bps = 0;
@@ -2203,7 +2199,7 @@ mcpet_status mcpet_run_device_noalloc(mcpet_scene* sc, const float* activity_dev
     return set_error(MCPET_ERR_ARG, "lowered loop caps are not available for the allocation-free run");
   const int mode = run_mode(sc, o);
   int block = transport_block_threads();
-  size_t smem = transport_dynamic_smem(P, block, kAlgorithmEvents, mode);
+  size_t smem = transport_dynamic_smem(P, block, kAlgorithmEvents);
   int bps = 0;
   CUDA_TRY(transport_occupancy(counters, kAlgorithmEvents, mode, block, smem, &bps));
   if (bps < 1) return set_error(MCPET_ERR_LIMIT, "transport kernel does not fit on an SM (smem %zu)", smem);

@@ -506,23 +506,26 @@ __global__ void plan_fill_kernel(const float* act, int nvox, int mode, int tpb, 
 /* ---------------------------------------------------------- launchers */
 
 /* Dynamic shared memory: spectrum, palette, shell scratch and the event
- * loop's per-thread state. */
-static size_t dynamic_smem(const TransportParams& P, int block, int algorithm, int mode, bool batch) {
+ * loop's per-thread fields (a single scene uses the fields before kCHist, a
+ * batch those before kCBx, a prompt-gamma scene all of them). */
+static size_t dynamic_smem(const TransportParams& P, int block, int algorithm, bool batch) {
   size_t s = 0;
   if (P.spectrum_in_shared) s += ((size_t)P.ne * 4 + 15) / 16 * 16;
   if (P.palette_in_shared) s += ((size_t)P.palette_in_shared * sizeof(PaletteEntry) + 15) / 16 * 16;
   s += (size_t)(P.max_shells > 0 ? P.max_shells : 1) * block * sizeof(float);
-  if (algorithm != kAlgorithmHistories)
-    s += (size_t)lane_words(mode, batch, algorithm == kAlgorithmEventsRecord) * block * sizeof(uint32_t);
+  if (algorithm != kAlgorithmHistories) {
+    const int fields = P.prompt_energy > 0.0f ? kCold : (batch ? kCBx : kColdSingle);
+    s += (size_t)fields * block * sizeof(uint32_t);
+  }
   return s;
 }
 
-size_t transport_dynamic_smem(const TransportParams& P, int block, int algorithm, int mode) {
-  return dynamic_smem(P, block, algorithm, mode, false);
+size_t transport_dynamic_smem(const TransportParams& P, int block, int algorithm) {
+  return dynamic_smem(P, block, algorithm, false);
 }
 
-size_t transport_batch_dynamic_smem(const TransportParams& P, int block, int mode) {
-  return dynamic_smem(P, block, kAlgorithmEvents, mode, true);
+size_t transport_batch_dynamic_smem(const TransportParams& P, int block) {
+  return dynamic_smem(P, block, kAlgorithmEvents, true);
 }
 
 int transport_block_threads() { return kBlock; }

@@ -28,7 +28,7 @@ constexpr int kTransportChained = 16;       /* single-scene launch of a batched 
                                                (programmatic dependent launch; seed read from the batch
                                                slot); plain event kernel, no loop caps */
 
-size_t transport_dynamic_smem(const TransportParams& P, int block, int algorithm, int mode);
+size_t transport_dynamic_smem(const TransportParams& P, int block, int algorithm);
 int transport_block_threads();
 cudaError_t transport_occupancy(bool counters, int algorithm, int mode, int block, size_t smem, int* blocks_per_sm);
 cudaError_t launch_transport(const TransportParams& P, const DeviceTables& T, const DeviceTallies& O,
@@ -40,7 +40,7 @@ cudaError_t launch_transport(const TransportParams& P, const DeviceTables& T, co
  * settings), bit 1 = every scene has the launch's phantom (grid, voxel keys,
  * palette, tables); those are then read from P and T (non-counting,
  * dose-free launches only) */
-size_t transport_batch_dynamic_smem(const TransportParams& P, int block, int mode);
+size_t transport_batch_dynamic_smem(const TransportParams& P, int block);
 constexpr int kBatchShareScanner = 1;
 constexpr int kBatchSharePhantom = 2;
 cudaError_t transport_batch_occupancy(bool counters, bool dose, int share, int mode, int block, size_t smem,

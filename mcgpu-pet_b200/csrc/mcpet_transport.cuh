@@ -83,15 +83,15 @@ __device__ __forceinline__ uint64_t claim_lane(unsigned long long* cursor) {
  * spread_lanes): the lane of rank r -- plans are ordered by decreasing work --
  * goes to warp r mod W of the grid's W warps, warps counted across the blocks
  * first, so that the longest lanes start on warps of their own on different
- * SMs (a thread's second lane after all first ones); later ones come from the
- * work queue, after those.  A lane is one serial chain of decays, and in a full warp it
+ * SMs; later ones come from the work queue, after the first gridDim *
+ * blockDim.  A lane is one serial chain of decays, and in a full warp it
  * waits for the rounds of 31 others: 25.8 us a decay with 32 of the hot
  * lanes of a 9^3 cube to a warp, 8.3 us with one (1e7 decays, 96 lanes of
  * 30458 decays each: 787 -> 253 ms).  Elsewhere the queue deals every lane,
  * in groups of consecutive ones that share voxels and scenes. */
-__device__ __forceinline__ uint64_t initial_lane(int slot) {
+__device__ __forceinline__ uint64_t initial_lane() {
   const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-  return ((threadIdx.x & 31) + 32 * slot) * warps + (uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  return (threadIdx.x & 31) * warps + (uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
 }
 
 /* The emitter of a lane: the last one whose first lane is not after it.  Eight
@@ -561,64 +561,23 @@ __global__ void __launch_bounds__(kBlock) transport_kernel(TransportParams P, De
  * point and first photon, the decay clock) lives in shared memory, laid out
  * [field][thread]. */
 
-/* Phases of a lane.  kPhEnd: photon 1 has left or was absorbed; kPhEndPair:
- * photon 2 (or a prompt gamma) has; kPhDecay: the next decay of the lane, or
- * (index < kLive) the next lane of the thread.  An absorbed or dropped photon
- * has energy -10. */
-enum : int { kPhDecay = 0, kPhStep = 1, kPhCompton = 2, kPhRayleigh = 3, kPhEnd = 4, kPhEndPair = 5, kPhDone = 6 };
-enum : int { kLive = -1, kNextLane = -2, kFirstLane = -3 };   /* index in kPhDecay */
-constexpr float kAbsorbed = -10.0f;
+enum : int { kPhDecay = 0, kPhStep = 1, kPhCompton = 2, kPhEnd = 3, kPhDone = 4 };  /* kPhCompton: any real scattering */
 
-/* Two lanes a thread: one in registers, one waiting in shared memory.  A
- * warp's phase vote then chooses among 64 photons for its 32 threads, and a
- * thread whose photon is in another phase exchanges it for the waiting one if
- * that is in the chosen phase (no photon ever leaves its thread): three wide
- * loads and stores and some forty instructions, against the hundreds of the
- * round.  5e7 decays of the head: 17.9e9 instructions of 10.8 threads become
- * 16.3e9 of 13.7; 1e9 decays 354 -> 328 ms.  Prompt-gamma variants
- * keep one lane a thread: their third photon needs the shared memory of two
- * thirds of a lane more, and only two blocks would be resident; and so do the
- * variants for measurements and tests, counters and lowered caps. */
-__host__ __device__ constexpr bool dual_lanes(int mode) { return !(mode & (kTransportPrompt | kTransportCaps)); }
-
-/* Words of a lane's state that a phase touches once a photon, in shared
- * memory (first word of each field).  Photon 1 at its exit takes the place of
- * the emission point and direction, which its end has used (a prompt gamma
- * needs the emission point once more). */
-struct LaneFields {
-  int o, d;              /* emission point and direction of photon 1: 3 + 3 */
-  int a;                 /* photon 1 at exit: position, direction (6), energy (-10 absorbed), state[, travel] */
-  int inv, left, vox;    /* lane: 1/rate (double, 2), remaining ps (2), voxel */
-  int trial, s0;         /* pending scattering: GCOa trials so far or Rayleigh pmax, GCOa's s0 (reference arithmetic) */
-  int hist, det;         /* batch: lane photons started, coincidences tallied */
-  int rx;                /* recording: RANECU state right before the pair's emission (2) */
-  int b;                 /* prompt gamma: photon 2 at exit, as a */
-  int words;             /* of one lane */
-  int saved;             /* of the waiting lane's registers */
+/* cold per-thread fields in shared memory */
+enum : int {
+  kCOx, kCOy, kCOz, kCDx, kCDy, kCDz,            /* emission point and direction of photon 1 */
+  kCAx, kCAy, kCAz, kCAu, kCAv, kCAw,            /* photon 1 at exit: position, direction */
+  kCAe, kCAt, kCAs,                              /* photon 1 energy (-10 absorbed), travel, state */
+  kCInvLo, kCInvHi, kCTLo, kCTHi, kCVox,         /* lane: 1/rate (double), remaining ps (u64), voxel */
+  kCRx, kCRy,                                    /* RANECU state right before the pair's emission */
+  kCTrial, kCS0,                                 /* pending Compton sampling: trials so far, its s0 */
+  kCHist, kCDet,                                 /* batch only: lane photons started, coincidences tallied */
+  kCPmax,                                        /* batch only: Rayleigh pmax of the pending interaction */
+  kCBx, kCBy, kCBz, kCBu, kCBv, kCBw,            /* prompt gamma only: photon 2 at exit: position, direction, */
+  kCBe, kCBt, kCBs,                              /* energy (-10 absorbed), travel, state */
+  kCold
 };
-__host__ __device__ constexpr LaneFields lane_fields(int mode, bool batch, bool record) {
-  const bool prompt = mode & kTransportPrompt, travel = !(mode & kTransportSinogramOnly);
-  LaneFields f = {};
-  f.o = 0;
-  f.d = 3;
-  f.a = prompt ? 6 : 0;
-  f.inv = f.a + 8 + (travel ? 1 : 0);
-  f.left = f.inv + 2;
-  f.vox = f.left + 2;
-  f.trial = f.vox + 1;
-  f.s0 = f.trial + 1;
-  f.hist = f.s0 + ((mode & kTransportFast) ? 0 : 1);
-  f.det = f.hist + 1;
-  f.rx = f.hist + (batch ? 2 : 0);
-  f.b = f.rx + (record ? 2 : 0);
-  f.words = f.b + (prompt ? 8 + (travel ? 1 : 0) : 0);
-  f.saved = 12 + (travel ? 1 : 0) + (batch ? 1 : 0);
-  return f;
-}
-constexpr int lane_words(int mode, bool batch, bool record) {
-  return lane_fields(mode, batch, record).words * (dual_lanes(mode) ? 2 : 1) +
-         (dual_lanes(mode) ? lane_fields(mode, batch, record).saved : 0);
-}
+constexpr int kColdSingle = kCHist;              /* fields a single-scene launch uses (the last ones need no room) */
 
 struct ColdState {
   uint32_t* base;
@@ -626,52 +585,20 @@ struct ColdState {
   __device__ __forceinline__ uint32_t& u(int f) const { return base[f * stride]; }
   __device__ __forceinline__ float f(int k) const { return __uint_as_float(base[k * stride]); }
   __device__ __forceinline__ void setf(int k, float v) const { base[k * stride] = __float_as_uint(v); }
-  __device__ __forceinline__ double real(int k) const {
-    return __hiloint2double((int)u(k + 1), (int)u(k));
+  __device__ __forceinline__ double inv_rate() const {
+    return __hiloint2double((int)u(kCInvHi), (int)u(kCInvLo));
   }
-  __device__ __forceinline__ void set_real(int k, double v) const {
-    u(k + 1) = (uint32_t)__double2hiint(v);
-    u(k) = (uint32_t)__double2loint(v);
+  __device__ __forceinline__ void set_inv_rate(double v) const {
+    u(kCInvHi) = (uint32_t)__double2hiint(v);
+    u(kCInvLo) = (uint32_t)__double2loint(v);
   }
-  __device__ __forceinline__ unsigned long long u64(int k) const {
-    return ((unsigned long long)u(k + 1) << 32) | u(k);
+  __device__ __forceinline__ unsigned long long t_left() const {
+    return ((unsigned long long)u(kCTHi) << 32) | u(kCTLo);
   }
-  __device__ __forceinline__ void set_u64(int k, unsigned long long v) const {
-    u(k + 1) = (uint32_t)(v >> 32);
-    u(k) = (uint32_t)v;
+  __device__ __forceinline__ void set_t_left(unsigned long long v) const {
+    u(kCTHi) = (uint32_t)(v >> 32);
+    u(kCTLo) = (uint32_t)v;
   }
-  __device__ __forceinline__ float3 vec(int k) const { return make_float3(f(k), f(k + 1), f(k + 2)); }
-  __device__ __forceinline__ void set_vec(int k, const float3& v) const {
-    setf(k, v.x);
-    setf(k + 1, v.y);
-    setf(k + 2, v.z);
-  }
-};
-
-/* The waiting lane's registers: rows of 16 bytes a thread, [row][thread], so
- * that a row is one wide load and store without bank conflicts, and single
- * words after them. */
-struct WaitingState {
-  uint32_t* base;       /* of the block */
-  __device__ __forceinline__ void exchange4(int row, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) const {
-    uint4* p = reinterpret_cast<uint4*>(base) + row * blockDim.x + threadIdx.x;
-    const uint4 t = *p;
-    *p = make_uint4(a, b, c, d);
-    a = t.x;
-    b = t.y;
-    c = t.z;
-    d = t.w;
-  }
-  __device__ __forceinline__ void exchange4(int row, float& a, float& b, float& c, float& d) const {
-    float4* p = reinterpret_cast<float4*>(base) + row * blockDim.x + threadIdx.x;
-    const float4 t = *p;
-    *p = make_float4(a, b, c, d);
-    a = t.x;
-    b = t.y;
-    c = t.z;
-    d = t.w;
-  }
-  __device__ __forceinline__ uint32_t& word(int k) const { return base[(12 + k) * blockDim.x + threadIdx.x]; }
 };
 
 
@@ -681,14 +608,9 @@ struct WaitingState {
 constexpr int kShareScanner = kBatchShareScanner;
 constexpr int kSharePhantom = kBatchSharePhantom;
 
-/* Resident blocks that the event kernel's registers are capped for: two lanes
- * a thread have the shared memory for 3 blocks of 256 (84 registers, no
- * spills), one lane has it for kMinBlocks. */
-constexpr int resident_blocks(int min_blocks, int mode) { return dual_lanes(mode) && min_blocks > 3 ? 3 : min_blocks; }
-
 template <bool kCount, int kMinBlocks = 1, bool kDevicePlan = false, bool kBatch = false, bool kRecord = false,
           bool kDose = false, int kShare = 0, int kMode = 0>
-__global__ void __launch_bounds__(kBlock, kCount ? kMinBlocks : resident_blocks(kMinBlocks, kMode)) transport_events_kernel(TransportParams P, DeviceTables T,
+__global__ void __launch_bounds__(kBlock, kMinBlocks) transport_events_kernel(TransportParams P, DeviceTables T,
                                                                               DeviceTallies O,
                                                                               const SceneSlot* __restrict__ slots,
                                                                               int n_slots) {
@@ -728,12 +650,7 @@ __global__ void __launch_bounds__(kBlock, kCount ? kMinBlocks : resident_blocks(
   }
   SharedScratch rn{reinterpret_cast<float*>(cursor) + threadIdx.x, (int)blockDim.x};
   cursor += (size_t)(P.max_shells > 0 ? P.max_shells : 1) * blockDim.x * sizeof(float);
-  constexpr LaneFields F = lane_fields(kMode, kBatch, kRecord);
-  constexpr bool kDual = dual_lanes(kMode) && !kCount;
-  constexpr bool kTravel = !(kMode & kModeSino);
-  const WaitingState saved{reinterpret_cast<uint32_t*>(cursor)};
-  if (kDual) cursor += (size_t)F.saved * blockDim.x * sizeof(uint32_t);
-  ColdState cold{reinterpret_cast<uint32_t*>(cursor) + threadIdx.x, (int)blockDim.x};   /* of the lane in registers */
+  const ColdState cold{reinterpret_cast<uint32_t*>(cursor) + threadIdx.x, (int)blockDim.x};
   {
     const int* src = reinterpret_cast<const int*>(T.compton);
     int* dst = reinterpret_cast<int*>(&cmp);
@@ -760,92 +677,44 @@ __global__ void __launch_bounds__(kBlock, kCount ? kMinBlocks : resident_blocks(
   /* dose: a block-shared copy of the material sums (global ones in a batch) */
   const bool dose_on = kDose && (kBatch || O.mat_dose || O.vox_dose);
 
-  /* the lane in registers */
+  /* hot per-thread state */
   Rng rng = {0, 0};
   int phase = kPhDecay;
-  int waiting = kPhDone;    /* phase of the thread's other lane */
-  int slot = 0;             /* which of the two is in registers */
-  /* a second lane a thread only where there are lanes for all first ones */
-  const unsigned threads = gridDim.x * blockDim.x;
-  const bool two = kDual && n_lanes > P.first_lane + threads;
+  bool lane_live = false;
+  bool first_claim = P.spread_lanes != 0;
   int which = 1;            /* photon of the pair being tracked */
+  bool fresh = false;       /* next step starts a new interaction-loop iteration */
+  bool escaped = false;
+  bool is_compton = true;   /* pending scattering: Compton (else Rayleigh) */
   PhotonState ph;
   ph.pos = make_float3(0.f, 0.f, 0.f);
   ph.dir = ph.pos;
   ph.energy = 0.f;
   ph.travel = 0.f;
   ph.state = 0;
-  int index = P.spread_lanes ? kFirstLane : kNextLane, mat_old = -1, mat0 = 0, steps = 0;
+  int index = 0, mat_old = -1, mat0 = 0, steps = 0;
   float mfp_w = 0.f, cax = 0.f, cbx = 0.f;
+  float4 rec_hi = make_float4(0.f, 0.f, 0.f, 0.f);   /* Rayleigh part of the last interaction record */
 
   /* photon emitted at ph.pos with ph.dir: set up its tracking */
   /* batch: the thread's totals for its current scene, added to that
    * scene's when the thread moves to another scene and at the end */
+  if (kBatch) {
+    cold.u(kCHist) = 0;
+    cold.u(kCDet) = 0;
+  }
+  cold.u(kCTrial) = 0;
   auto flush_lane = [&]() {
     if (!kBatch) return;
-    const unsigned long long h = cold.u(F.hist), c = cold.u(F.det);
+    const unsigned long long h = cold.u(kCHist), c = cold.u(kCDet);
     if (h) atomicAdd(slots[scene].O.histories, h);
     if (c && slots[scene].O.coincidences) atomicAdd(slots[scene].O.coincidences, c);
-    cold.u(F.hist) = 0;
-    cold.u(F.det) = 0;
+    cold.u(kCHist) = 0;
+    cold.u(kCDet) = 0;
   };
-
-  /* the lane in registers changes places with the waiting one (the material's
-   * coefficients are loaded again instead) */
-  auto exchange_lanes = [&]() {
-    uint32_t misc = (uint32_t)phase | (uint32_t)which << 3 | (uint32_t)ph.state << 5 | (uint32_t)mat0 << 7 |
-                    (uint32_t)steps << 11;   /* at most 2^20 + 1 */
-    uint32_t at = (uint32_t)index, rx = (uint32_t)rng.x, ry = (uint32_t)rng.y;
-    waiting = phase;
-    saved.exchange4(0, ph.pos.x, ph.pos.y, ph.pos.z, ph.energy);
-    saved.exchange4(1, ph.dir.x, ph.dir.y, ph.dir.z, mfp_w);
-    saved.exchange4(2, rx, ry, at, misc);
-    if (kTravel) {
-      const float t = __uint_as_float(saved.word(0));
-      saved.word(0) = __float_as_uint(ph.travel);
-      ph.travel = t;
-    }
-    if (kBatch) {
-      const int t = (int)saved.word(kTravel ? 1 : 0);
-      saved.word(kTravel ? 1 : 0) = (uint32_t)scene;
-      scene = t;
-    }
-    rng.x = (int)rx;
-    rng.y = (int)ry;
-    index = (int)at;
-    phase = (int)(misc & 7u);
-    which = (int)(misc >> 3 & 3u);
-    ph.state = (int)(misc >> 5 & 3u);
-    mat0 = (int)(misc >> 7 & 15u);
-    steps = (int)(misc >> 11);
-    mat_old = -2;
-    cold.base += slot ? -F.words * (int)blockDim.x : F.words * (int)blockDim.x;
-    slot ^= 1;
-  };
-  if (kBatch) {
-    cold.u(F.hist) = 0;
-    cold.u(F.det) = 0;
-  }
-  cold.u(F.trial) = 0;
-  if (kDual) {
-    /* the waiting lane starts as the other, or done */
-    waiting = two ? kPhDecay : kPhDone;
-    uint32_t zero = 0, at = (uint32_t)index, misc = (uint32_t)waiting | 1u << 3, rx = 0, ry = 0;
-    float z0 = 0, z1 = 0, z2 = 0, z3 = 0;
-    saved.exchange4(0, z0, z1, z2, z3);
-    z0 = z1 = z2 = z3 = 0;
-    saved.exchange4(1, z0, z1, z2, z3);
-    saved.exchange4(2, rx, ry, at, misc);
-    for (int k = 12; k < F.saved; ++k) saved.word(k - 12) = zero;
-    if (kBatch) {
-      cold.u(F.words + F.hist) = 0;
-      cold.u(F.words + F.det) = 0;
-    }
-    cold.u(F.words + F.trial) = 0;
-  }
 
   /* (the scenes of a batch share the energy grid: e0 and ide are P's) */
-  auto start_photon = [&](const DeviceTables& TW, const TransportParams& PW, float energy) {
+  auto start_photon = [&](const DeviceTables& TW, float energy) {
     ph.energy = energy;
     ph.travel = 0.0f;
     ph.state = 0;
@@ -853,73 +722,61 @@ __global__ void __launch_bounds__(kBlock, kCount ? kMinBlocks : resident_blocks(
     Counting<kCount>::add(cnt.photons, 1);
     if ((kMode & kModePrompt) && (index < 0 || index >= P.n_e - 1)) {   /* energy outside the tables */
       Counting<true>::add(cnt.guard, 1);
-      ph.energy = kAbsorbed;
-      phase = which == 1 ? kPhEnd : kPhEndPair;
+      escaped = false;
+      phase = kPhEnd;
       return;
     }
     float2 w = __ldg(reinterpret_cast<const float2*>(TW.woodcock) + index);
     mfp_w = w.x + ph.energy * w.y;
     mat_old = -1;
     steps = 0;
-    /* a photon that starts within EPS of the phantom's faces has left it
-     * (MCGPU-PET_kernel.cu:313-317); where a photon scatters, its step has just
-     * found it inside */
-    if (locate(PW, ph.pos.x, ph.pos.y, ph.pos.z) >= 0) phase = kPhStep;
-    else phase = which == 1 ? kPhEnd : kPhEndPair;
+    fresh = true;
+    phase = kPhStep;
     Counting<kCount>::add(cnt.majorant, 1);
   };
 
   for (;;) {
-    /* phases of the thread's lanes, and the threads that have one in each */
-    const unsigned has = (1u << phase) | (kDual ? 1u << waiting : 0u);
-    const unsigned m_step = __ballot_sync(0xffffffffu, has & (1u << kPhStep));
-    const unsigned m_cmp = __ballot_sync(0xffffffffu, has & (1u << kPhCompton));
-    const unsigned m_ray = __ballot_sync(0xffffffffu, has & (1u << kPhRayleigh));
-    const unsigned m_end = __ballot_sync(0xffffffffu, has & (1u << kPhEnd));
-    const unsigned m_pair = __ballot_sync(0xffffffffu, has & (1u << kPhDecay | 1u << kPhEndPair));
-    if (!(m_step | m_cmp | m_ray | m_end | m_pair)) break;
-    /* phase of this round: the others wait until enough threads need them;
-     * Woodcock steps fill the rest.  Rayleigh lanes (GRAa) join a round with
-     * Compton lanes only when at least quorum_rayleigh of them wait, so that
-     * most rounds run one sampler. */
-    const int n_cmp = __popc(m_cmp | m_ray), n_end = __popc(m_end), n_pair = __popc(m_pair);
-    const bool ray_now = !m_cmp || __popc(m_ray) >= P.quorum_rayleigh;
-    int sel;
-    if (n_cmp >= P.quorum_scatter) sel = kPhCompton;
-    else if (n_pair >= P.quorum_pair) sel = kPhEndPair;
-    else if (n_end >= P.quorum_pair) sel = kPhEnd;
-    else if (m_step) sel = kPhStep;
-    else sel = n_cmp >= max(n_pair, n_end) ? kPhCompton : n_pair >= n_end ? kPhEndPair : kPhEnd;
-    if (kDual) {
-      unsigned want = 1u << sel;
-      if (sel == kPhEndPair) want |= 1u << kPhDecay;
-      if (sel == kPhCompton && ray_now) want |= 1u << kPhRayleigh;
-      if (!(want >> phase & 1u) && (want >> waiting & 1u)) exchange_lanes();
-    }
+    const unsigned m_dec = __ballot_sync(0xffffffffu, phase == kPhDecay);
+    const unsigned m_step = __ballot_sync(0xffffffffu, phase == kPhStep);
+    const unsigned m_cmp = __ballot_sync(0xffffffffu, phase == kPhCompton);
+    const unsigned m_end = __ballot_sync(0xffffffffu, phase == kPhEnd);
+    if (!(m_dec | m_step | m_cmp | m_end)) break;
     const TransportParams& PS = kBatch ? slots[scene].P : P;
     /* phantom (grid, voxels, tables) and scanner (detector, sinogram) of the
      * current lane's scene */
     const TransportParams& PG = (kBatch && !(kShare & kSharePhantom)) ? slots[scene].P : P;
     const DeviceTables& TG = (kBatch && !(kShare & kSharePhantom)) ? slots[scene].T : T;
     const TransportParams& PD = (kBatch && !(kShare & kShareScanner)) ? slots[scene].P : P;
+    /* phase of this round: scattering and pair bookkeeping wait until enough
+     * lanes need them; Woodcock steps fill the rest */
+    const int n_cmp = __popc(m_cmp), n_pair = __popc(m_end | m_dec);
+    int sel;
+    if (n_cmp >= P.quorum_scatter) sel = 0;
+    else if (n_pair >= P.quorum_pair) sel = 1;
+    else if (m_step) sel = 2;
+    else sel = (n_cmp >= n_pair) ? 0 : 1;
 
-    if (sel == kPhCompton) {
+    if (sel == 0) {
       /* ---- real scattering: Compton (MCGPU-PET_kernel.cu:351-373) or
-       * Rayleigh (:375-387), then the common direction update.  The Compton lanes repeat the envelope part of GCOa's first stage
+       * Rayleigh (:375-387), then the common direction update.  Rayleigh
+       * lanes (GRAa) join a round with Compton lanes only when at least
+       * quorum_rayleigh of them wait, so that most rounds run one sampler.
+       * The Compton lanes repeat the envelope part of GCOa's first stage
        * until at most an eighth of them lacks a candidate, then evaluate the
        * shells of all candidates at once, and so on until at most an eighth
        * is still rejected; those keep their phase and go
        * on in a later round, with the lanes that arrive meanwhile, instead of
        * holding the warp in the rejection loop (each lane draws its random
        * numbers in the same order either way) */
-      const unsigned m_c = __ballot_sync(0xffffffffu, phase == kPhCompton);
-      if (phase == kPhCompton || (phase == kPhRayleigh && ray_now)) {
-        const bool is_compton = phase == kPhCompton;
+      const unsigned m_ray = __ballot_sync(0xffffffffu, phase == kPhCompton && !is_compton);
+      const unsigned m_c = m_cmp & ~m_ray;
+      const bool ray_now = (m_cmp == m_ray) || (__popc(m_ray) >= P.quorum_rayleigh);
+      if (phase == kPhCompton && (is_compton || ray_now)) {
         double costh = 0.0;
         bool ok = false, pending = false;
         float e = ph.energy;
         if (__builtin_expect(is_compton, 1)) {
-          uint32_t trials = cold.u(F.trial);
+          uint32_t trials = cold.u(kCTrial);
           float s0;
           if (kMode & kModeFast) {
             /* balanced lanes: the bin's bound of the normaliser */
@@ -928,9 +785,9 @@ __global__ void __launch_bounds__(kBlock, kCount ? kMinBlocks : resident_blocks(
             s0 = s0_ann[mat0];
           } else if (trials == 0) {
             s0 = compton_s0(e, mat0, cmp);
-            cold.setf(F.s0, s0);
+            cold.setf(kCS0, s0);
           } else {
-            s0 = cold.f(F.s0);
+            s0 = cold.f(kCS0);
           }
           float tau = 0.f, s = 0.f, u = 0.f;
           double cdt1 = 0.0;
@@ -950,28 +807,26 @@ __global__ void __launch_bounds__(kBlock, kCount ? kMinBlocks : resident_blocks(
             if (8 * __popc(__ballot_sync(m_c, !accepted && !tripped)) <= __popc(m_c)) break;
           }
           if (accepted) {
-            cold.u(F.trial) = 0;
+            cold.u(kCTrial) = 0;
             costh = 1.0 - cdt1;
             ok = compton_doppler<(kMode & kModeFast) != 0>(rng, e, mat0, cmp, rn, tau, s, costh,
                                                            rejections_cap<kMode>(P));
           } else if (tripped) {
-            cold.u(F.trial) = 0;
+            cold.u(kCTrial) = 0;
           } else {
-            cold.u(F.trial) = trials;
+            cold.u(kCTrial) = trials;
             pending = true;
           }
         } else {
-          const float pmax = cold.f(F.trial);
-          cold.u(F.trial) = 0;
-          ok = sample_rayleigh(rng, e, mat0, pmax, T.rayleigh, costh,
+          ok = sample_rayleigh(rng, e, mat0, kBatch ? cold.f(kCPmax) : rec_hi.z, T.rayleigh, costh,
                                rejections_cap<kMode>(P));
         }
         if (pending) {
           /* next trial in a later scattering round */
         } else if (__builtin_expect(!ok, 0)) {
           Counting<true>::add(cnt.guard, 1);
-          ph.energy = kAbsorbed;
-          phase = which == 1 ? kPhEnd : kPhEndPair;
+          escaped = false;
+          phase = kPhEnd;
         } else {
           const float e_before = ph.energy;
           ph.energy = e;
@@ -990,92 +845,103 @@ __global__ void __launch_bounds__(kBlock, kCount ? kMinBlocks : resident_blocks(
               mat_old = -2;
               ph.state = (ph.state == 0) ? 1 : 3;
               Counting<kCount>::add(cnt.majorant, 1);
+              fresh = true;
               phase = kPhStep;
             } else {
-              ph.energy = kAbsorbed;
-              phase = which == 1 ? kPhEnd : kPhEndPair;
+              escaped = false;
+              phase = kPhEnd;
             }
           } else {
             ph.state = (ph.state == 0) ? 2 : 3;
             Counting<kCount>::add(cnt.rayleigh, 1);
+            fresh = true;
             phase = kPhStep;
           }
         }
       }
-    } else if (sel == kPhEnd) {
-      /* ---- end of photon 1: keep it, emit photon 2 (MCGPU-PET_kernel.cu:417-442) */
+    } else if (sel == 1) {
+      /* ---- end of a photon: hand over to the second photon, or close the
+       * pair (MCGPU-PET_kernel.cu:417-442); then the next decay */
       if (phase == kPhEnd) {
-        const float3 d0 = cold.vec(F.d), origin = cold.vec(F.o);
-        cold.set_vec(F.a, ph.pos);
-        cold.set_vec(F.a + 3, ph.dir);
-        cold.setf(F.a + 6, ph.energy);
-        cold.u(F.a + 7) = (uint32_t)ph.state;
-        if (kTravel) cold.setf(F.a + 8, ph.travel);
-        emit_second<(kMode & kModeFast) != 0>(rng, background, d0, ph.dir);
-        ph.pos = origin;
-        which = 2;
-        start_photon(TG, PG, kAnnihilation);
-      }
-    } else if (sel == kPhEndPair) {
-      /* ---- end of photon 2 (or of a prompt gamma): close the pair
-       * (MCGPU-PET_kernel.cu:417-442) */
-      if (phase == kPhEndPair) {
-        /* end of photon 2: its pair with photon 1; end of a prompt gamma
-         * (which == 3): its pairs with photons 1 and 2, spurious */
-        const bool prompt = (kMode & kModePrompt) && PS.prompt_energy > 0.0f;
-        if (which == 2 && prompt) {
-          cold.set_vec(F.b, ph.pos);
-          cold.set_vec(F.b + 3, ph.dir);
-          cold.setf(F.b + 6, ph.energy);
-          cold.u(F.b + 7) = (uint32_t)ph.state;
-          if (kTravel) cold.setf(F.b + 8, ph.travel);
-        }
-        const bool spurious = (kMode & kModePrompt) && which == 3;
-        const int partners = spurious ? 2 : 1;
-        phase = kPhDecay;
-        index = kLive;
-#pragma unroll 1
-        for (int k = 0; k < partners; ++k) {
-          const int f = k == 0 ? F.a : F.b;   /* photon 1 or photon 2 */
-          const float ea = cold.f(f + 6);
-          if (ph.energy > -0.5f && ea > -0.5f) {
-            PhotonState a;
-            a.pos = cold.vec(f);
-            a.dir = cold.vec(f + 3);
-            a.energy = ea;
-            a.travel = kTravel ? cold.f(f + 8) : 0.0f;
-            a.state = (int)cold.u(f + 7);
-            const bool pass = spurious ? (PD.tally_type != 1)
-                                       : (PD.tally_type == 0) || (PD.tally_type == 1 && ph.state == 0 && a.state == 0) ||
-                                             (PD.tally_type == 2 && (ph.state != 0 || a.state != 0));
-            if (pass) {
-              unsigned long long det = 0;
-              detect_pair<kCount, kRecord, !(kMode & kModeSino), (kMode & kModeFast) != 0>(
-                  rng, PD, make_float3(PD.cx, PD.cy, PD.cz), kBatch ? slots[scene].O : O, spec_sh, (int)cold.u(F.vox), cold.u64(F.left), ph, a,
-                  cnt, det, kRecord ? make_int2((int)cold.u(F.rx), (int)cold.u(F.rx + 1)) : make_int2(0, 0),
-                  spurious);
-              if (kBatch) cold.u(F.det) += (uint32_t)det;
-              else detected += det;
+        if (which == 1) {
+          if (escaped) {
+            cold.setf(kCAx, ph.pos.x); cold.setf(kCAy, ph.pos.y); cold.setf(kCAz, ph.pos.z);
+            cold.setf(kCAu, ph.dir.x); cold.setf(kCAv, ph.dir.y); cold.setf(kCAw, ph.dir.z);
+            cold.setf(kCAe, ph.energy); cold.setf(kCAt, ph.travel);
+            cold.u(kCAs) = (uint32_t)ph.state;
+          } else {
+            cold.setf(kCAe, -10.0f);
+          }
+          const float3 d0 = make_float3(cold.f(kCDx), cold.f(kCDy), cold.f(kCDz));
+          emit_second<(kMode & kModeFast) != 0>(rng, background, d0, ph.dir);
+          ph.pos = make_float3(cold.f(kCOx), cold.f(kCOy), cold.f(kCOz));
+          which = 2;
+          start_photon(TG, kAnnihilation);
+        } else {
+          /* end of photon 2: its pair with photon 1; end of a prompt gamma
+           * (which == 3): its pairs with photons 1 and 2, spurious */
+          const bool prompt = (kMode & kModePrompt) && PS.prompt_energy > 0.0f;
+          if (which == 2 && prompt) {
+            if (escaped) {
+              cold.setf(kCBx, ph.pos.x); cold.setf(kCBy, ph.pos.y); cold.setf(kCBz, ph.pos.z);
+              cold.setf(kCBu, ph.dir.x); cold.setf(kCBv, ph.dir.y); cold.setf(kCBw, ph.dir.z);
+              cold.setf(kCBe, ph.energy); cold.setf(kCBt, ph.travel);
+              cold.u(kCBs) = (uint32_t)ph.state;
+            } else {
+              cold.setf(kCBe, -10.0f);
             }
           }
-        }
-        if (which == 2 && prompt && (PS.prompt_yield >= 1.0f || ranecu(rng) < PS.prompt_yield)) {
-          /* the prompt gamma: isotropic from the decay point */
-          emit_isotropic(rng, ph.dir);
-          ph.pos = cold.vec(F.o);
-          which = 3;
-          if (kBatch) cold.u(F.hist) += 1;
-          else histories += 1;
-          start_photon(TG, PG, PS.prompt_energy);
+          const bool spurious = (kMode & kModePrompt) && which == 3;
+          const int partners = spurious ? 2 : 1;
+#pragma unroll 1
+          for (int k = 0; k < partners; ++k) {
+            const int f = k == 0 ? kCAx : kCBx;   /* photon 1 or photon 2: 9 fields in the same order */
+            const float ea = cold.f(f + (kCAe - kCAx));
+            if (escaped && ea > -0.5f) {
+              PhotonState a;
+              a.pos = make_float3(cold.f(f), cold.f(f + 1), cold.f(f + 2));
+              a.dir = make_float3(cold.f(f + 3), cold.f(f + 4), cold.f(f + 5));
+              a.energy = ea;
+              a.travel = cold.f(f + (kCAt - kCAx));
+              a.state = (int)cold.u(f + (kCAs - kCAx));
+              const bool pass = spurious ? (PD.tally_type != 1)
+                                         : (PD.tally_type == 0) || (PD.tally_type == 1 && ph.state == 0 && a.state == 0) ||
+                                               (PD.tally_type == 2 && (ph.state != 0 || a.state != 0));
+              if (pass) {
+                unsigned long long det = 0;
+                detect_pair<kCount, kRecord, !(kMode & kModeSino), (kMode & kModeFast) != 0>(rng, PD, make_float3(PD.cx, PD.cy, PD.cz),
+                                                                  kBatch ? slots[scene].O : O,
+                                             spec_sh, (int)cold.u(kCVox),
+                                             cold.t_left(), ph, a, cnt, det,
+                                             kRecord ? make_int2((int)cold.u(kCRx), (int)cold.u(kCRy))
+                                                     : make_int2(0, 0),
+                                             spurious);
+                if (kBatch) cold.u(kCDet) += (uint32_t)det;
+                else detected += det;
+              }
+            }
+          }
+          if (which == 2 && prompt && (PS.prompt_yield >= 1.0f || ranecu(rng) < PS.prompt_yield)) {
+            /* the prompt gamma: isotropic from the decay point */
+            emit_isotropic(rng, ph.dir);
+            ph.pos = make_float3(cold.f(kCOx), cold.f(kCOy), cold.f(kCOz));
+            which = 3;
+            if (kBatch) cold.u(kCHist) += 1;
+            else histories += 1;
+            start_photon(TG, PS.prompt_energy);
+          } else {
+            phase = kPhDecay;
+          }
         }
       }
       /* ---- next decay of the lane, or the next lane (MCGPU-PET_kernel.cu:259-298) */
       if (phase == kPhDecay) {
         for (;;) {
-          if (__builtin_expect(index != kLive, 0)) {   /* rare branches hinted: cold code out of the hot paths */
+          if (__builtin_expect(!lane_live, 0)) {   /* rare branches hinted: cold code out of the hot paths */
             uint64_t lane = P.first_lane;
-            if (index == kFirstLane) lane += initial_lane(slot);
-            else lane += claim_lane(O.lane_cursor) + (P.spread_lanes ? (two ? 2 * threads : threads) : 0);
+            if (__builtin_expect(first_claim, 0)) lane += initial_lane();
+            else lane += claim_lane(O.lane_cursor) + (P.spread_lanes ? gridDim.x * blockDim.x : 0);
+            first_claim = false;
             if (lane >= n_lanes) {
               phase = kPhDone;
               break;
@@ -1100,38 +966,37 @@ __global__ void __launch_bounds__(kBlock, kCount ? kMinBlocks : resident_blocks(
             const TransportParams& PN = kBatch ? slots[scene].P : P;
             const int seed = (!kBatch && (kMode & kModeChain)) ? __ldg(O.seed_word) : PN.seed;
             rng = rng_stream(seed, __ldg(&em->stream_base) + (local - __ldg(&em->first_lane)));
-            cold.set_real(F.inv, __ldg(&em->inv_rate));
-            cold.set_u64(F.left, PN.acq_ps);
-            cold.u(F.vox) = __ldg(&em->voxel);
-            index = kLive;
+            cold.set_inv_rate(__ldg(&em->inv_rate));
+            cold.set_t_left(PN.acq_ps);
+            cold.u(kCVox) = __ldg(&em->voxel);
+            lane_live = true;
             Counting<kCount>::add(cnt.lanes, 1);
           }
           const TransportParams& PN = kBatch ? slots[scene].P : P;
-          double inv_act = cold.real(F.inv);
-          unsigned long long t_left = cold.u64(F.left);
+          double inv_act = cold.inv_rate();
+          unsigned long long t_left = cold.t_left();
           const unsigned long long dt_ps = decay_interval<(kMode & kModeFast) != 0>(rng, inv_act, PN.inv_mean_life);
           if (__builtin_expect(!(dt_ps < t_left), 0)) {
-            index = kNextLane;
+            lane_live = false;
             continue;
           }
-          cold.set_u64(F.left, t_left - dt_ps);
+          cold.set_t_left(t_left - dt_ps);
           if (kBatch) {
-            cold.u(F.hist) += 2;
-            if (cold.u(F.hist) >= 0x80000000u) flush_lane();   /* keep the 32-bit word from wrapping */
+            cold.u(kCHist) += 2;
+            if (cold.u(kCHist) >= 0x80000000u) flush_lane();   /* keep the 32-bit word from wrapping */
           }
           else histories += 2;
-          cold.set_real(F.inv, inv_act);
-          const int voxel = (int)cold.u(F.vox);
+          cold.set_inv_rate(inv_act);
+          const int voxel = (int)cold.u(kCVox);
           if (kRecord) {
-            cold.u(F.rx) = (uint32_t)rng.x;
-            cold.u(F.rx + 1) = (uint32_t)rng.y;
+            cold.u(kCRx) = (uint32_t)rng.x;
+            cold.u(kCRy) = (uint32_t)rng.y;
           }
           emit_first(rng, PN, voxel % PN.nx, (voxel / PN.nx) % PN.ny, voxel / (PN.nx * PN.ny), ph.pos, ph.dir);
-          cold.set_vec(F.o, ph.pos);
-          cold.set_vec(F.d, ph.dir);
+          cold.setf(kCOx, ph.pos.x); cold.setf(kCOy, ph.pos.y); cold.setf(kCOz, ph.pos.z);
+          cold.setf(kCDx, ph.dir.x); cold.setf(kCDy, ph.dir.y); cold.setf(kCDz, ph.dir.z);
           which = 1;
-          start_photon((kBatch && !(kShare & kSharePhantom)) ? slots[scene].T : T,
-                       (kBatch && !(kShare & kSharePhantom)) ? slots[scene].P : P, kAnnihilation);
+          start_photon((kBatch && !(kShare & kSharePhantom)) ? slots[scene].T : T, kAnnihilation);
           break;
         }
       }
@@ -1142,20 +1007,30 @@ __global__ void __launch_bounds__(kBlock, kCount ? kMinBlocks : resident_blocks(
       for (;;) {
         if (phase == kPhStep) {
           const float E = ph.energy;
-          {
+          bool go = true;
+          if (fresh) {
+            fresh = false;
+            if (locate(PG, ph.pos.x, ph.pos.y, ph.pos.z) < 0) {
+              escaped = true;
+              phase = kPhEnd;
+              go = false;
+            }
+          }
+          if (go) {
             float step = -(mfp_w)*logf(ranecu(rng));
-            if (kTravel) ph.travel += step;
+            ph.travel += step;
             ph.pos.x += step * ph.dir.x;
             ph.pos.y += step * ph.dir.y;
             ph.pos.z += step * ph.dir.z;
             const int vox = locate(PG, ph.pos.x, ph.pos.y, ph.pos.z);
             if (vox < 0) {
-              phase = which == 1 ? kPhEnd : kPhEndPair;
+              escaped = true;
+              phase = kPhEnd;
             } else if (__builtin_expect((unsigned long long)vox >= (unsigned long long)PG.n_voxels ||
                                             ++steps > steps_cap<kMode>(P), 0)) {
               Counting<true>::add(cnt.guard, 1);
-              ph.energy = kAbsorbed;
-              phase = which == 1 ? kPhEnd : kPhEndPair;
+              escaped = false;
+              phase = kPhEnd;
             } else {
               const uint32_t key = TG.vox16 ? (uint32_t)__ldg(&TG.vox16[vox]) : __ldg(&TG.vox32[vox]);
               const PaletteEntry pe = (kBatch && !(kShare & kSharePhantom)) ? TG.palette[key] : pal[key];
@@ -1179,15 +1054,19 @@ __global__ void __launch_bounds__(kBlock, kCount ? kMinBlocks : resident_blocks(
                 prob += mfp_density * (cc.x + E * cc.y);
                 if (__builtin_expect(randno < prob, 1)) {
                   phase = kPhCompton;
+                  is_compton = true;
                 } else {
-                  const float4 rec_hi = __ldg(reinterpret_cast<const float4*>(rec) + 1);
+                  rec_hi = __ldg(reinterpret_cast<const float4*>(rec) + 1);
                   prob += mfp_density * (rec_hi.x + E * rec_hi.y);
                   if (randno < prob) {
-                    phase = kPhRayleigh;
-                    cold.setf(F.trial, rec_hi.z);
+                    phase = kPhCompton;
+                    is_compton = false;
+                    /* a batch keeps pmax in shared memory (fewer live registers) */
+                    if (kBatch) cold.setf(kCPmax, rec_hi.z);
                   } else {
-                    ph.energy = kAbsorbed;
-                    phase = which == 1 ? kPhEnd : kPhEndPair;
+                    index = -11;
+                    escaped = false;
+                    phase = kPhEnd;
                     Counting<kCount>::add(cnt.photo, 1);
                     if (dose_on) {
                       const DoseSink ds{kBatch ? slots[scene].O.mat_dose : (O.mat_dose ? mdose_sh : nullptr),
@@ -1211,10 +1090,6 @@ __global__ void __launch_bounds__(kBlock, kCount ? kMinBlocks : resident_blocks(
   if (kBatch || (kMode & kModeChain)) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (kBatch) {
     flush_lane();
-    if (kDual) {
-      exchange_lanes();
-      flush_lane();
-    }
   } else {
     atomicAdd(O.histories, histories);
     if (detected) atomicAdd(O.coincidences, detected);
