@@ -420,8 +420,8 @@ __device__ __forceinline__ float compton_s0(float E, int mat, const ComptonTable
  * and s0 is its value at pi or a bound of that), so a draw above the
  * Klein-Nishina factor, by a margin far over the rounding of both sums, is
  * rejected.  The shell part evaluates the sum and the test itself for the
- * draws that are left.  At 511 keV the first rejects 4 in 10 trials and the
- * second 1 in 50, so that callers repeat the cheap part until (nearly) all
+ * draws that are left.  At 511 keV in water the first rejects 1 in 4 trials
+ * and the second fewer than 1 in 1000, so that callers repeat the cheap part until (nearly) all
  * their lanes have a candidate and evaluate the shells -- a square root and an
  * exponential each -- once a sampling, with full warps.  A trial draws the
  * same random numbers whatever part ends it, and whether the trials of one
