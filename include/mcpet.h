@@ -498,6 +498,12 @@ mcpet_status mcpet_probe_detector(const mcpet_scene* scene, int n, const float* 
 mcpet_status mcpet_probe_compton(const mcpet_scene* scene, int n, const float* energy_in,
                                  const int32_t* mat, const int32_t* seeds_in, float* energy_out,
                                  double* costh_out, int32_t* seeds_out);
+/* The rejection test of a Compton trial with E'/E = tau and draw u (GCOa
+ * :1436-1451): out[i] bit 0 set when the early part (before the sum over the
+ * shells) rejects, bit 1 when the whole test does. */
+mcpet_status mcpet_probe_compton_test(const mcpet_scene* scene, int n, const float* energy,
+                                      const int32_t* mat, const float* tau, const float* u,
+                                      int32_t* out);
 mcpet_status mcpet_probe_rayleigh(const mcpet_scene* scene, int n, const float* energy_in,
                                   const int32_t* mat, const float* pmax, const int32_t* seeds_in,
                                   double* costh_out, int32_t* seeds_out);

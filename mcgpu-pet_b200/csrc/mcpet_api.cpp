@@ -2343,6 +2343,30 @@ mcpet_status mcpet_probe_compton(const mcpet_scene* sc, int n, const float* ener
   return MCPET_OK;
 }
 
+mcpet_status mcpet_probe_compton_test(const mcpet_scene* sc, int n, const float* energy, const int32_t* mat,
+                                      const float* tau, const float* u, int32_t* out) {
+  if (!sc || n <= 0 || !energy || !mat || !tau || !u || !out)
+    return set_error(MCPET_ERR_ARG, "invalid probe arguments");
+  for (int i = 0; i < n; ++i)
+    if (mat[i] < 0 || mat[i] >= kMaxMaterials || !sc->material_loaded[mat[i]])
+      return set_error(MCPET_ERR_ARG, "material %d not loaded", mat[i]);
+  mcpet_status s = probe_device();
+  if (s != MCPET_OK) return s;
+  DBuf<ComptonTable> tab;
+  DBuf<float> de, dt, du;
+  DBuf<int> dm, dout;
+  CUDA_TRY(tab.alloc(1, &sc->compton));
+  CUDA_TRY(de.alloc(n, energy));
+  CUDA_TRY(dm.alloc(n, mat));
+  CUDA_TRY(dt.alloc(n, tau));
+  CUDA_TRY(du.alloc(n, u));
+  CUDA_TRY(dout.alloc(n));
+  CUDA_TRY(launch_probe_compton_test(tab.p, n, de.p, dm.p, dt.p, du.p, dout.p, nullptr));
+  CUDA_TRY(cudaDeviceSynchronize());
+  CUDA_TRY(cudaMemcpy(out, dout.p, sizeof(int) * n, cudaMemcpyDeviceToHost));
+  return MCPET_OK;
+}
+
 mcpet_status mcpet_probe_rayleigh(const mcpet_scene* sc, int n, const float* energy_in, const int32_t* mat,
                                   const float* pmax, const int32_t* seeds_in, double* costh_out, int32_t* seeds_out) {
   if (!sc || n <= 0 || !energy_in || !mat || !pmax || !seeds_in || !costh_out || !seeds_out)

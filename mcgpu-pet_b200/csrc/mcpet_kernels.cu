@@ -104,6 +104,30 @@ __global__ void probe_compton_kernel(const ComptonTable* tab, int n, float* ener
   seeds[i] = make_int2(r.x, r.y);
 }
 
+/* Both parts of a Compton trial's rejection test for given tau and draw u:
+ * bit 0 when compton_refused rejects, bit 1 when compton_shells does. */
+__global__ void probe_compton_test_kernel(const ComptonTable* tab, int n, const float* energy, const int* mat,
+                                          const float* tau, const float* u, int* out) {
+  __shared__ ComptonTable cmp;
+  extern __shared__ float4 dyn_smem[];
+  {
+    const int* src = reinterpret_cast<const int*>(tab);
+    int* dst = reinterpret_cast<int*>(&cmp);
+    for (int i = threadIdx.x; i < (int)(sizeof(ComptonTable) / 4); i += blockDim.x) dst[i] = src[i];
+  }
+  __syncthreads();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  SharedScratch rn{reinterpret_cast<float*>(dyn_smem) + threadIdx.x, (int)blockDim.x};
+  const float e = energy[i], t = tau[i];
+  double cdt1 = (double)(1.f - t) / (((double)t) * ((double)e) * 1.956951306108245e-6);
+  if (cdt1 > 2.0) cdt1 = 1.99999999;
+  float s, num, den;
+  const bool early = compton_refused(e, t, u[i], num, den);
+  const bool kept = compton_shells(e, mat[i], cmp, rn, compton_s0(e, mat[i], cmp), t, cdt1, u[i], num, den, s);
+  out[i] = (early ? 1 : 0) | (kept ? 0 : 2);
+}
+
 __global__ void probe_rayleigh_kernel(RayleighRows R, int n, const float* energy, const int* mat, const float* pmax,
                                       int2* seeds, double* costh) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -657,6 +681,13 @@ cudaError_t launch_probe_compton(const ComptonTable* tab, int n, float* energy, 
                                  double* costh, cudaStream_t s) {
   size_t smem = (size_t)kMaxShells * 128 * sizeof(float);
   probe_compton_kernel<<<(n + 127) / 128, 128, smem, s>>>(tab, n, energy, mat, seeds, costh, kMaxShells);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_probe_compton_test(const ComptonTable* tab, int n, const float* energy, const int* mat,
+                                      const float* tau, const float* u, int* out, cudaStream_t s) {
+  const size_t smem = (size_t)kMaxShells * 128 * sizeof(float);
+  probe_compton_test_kernel<<<(n + 127) / 128, 128, smem, s>>>(tab, n, energy, mat, tau, u, out);
   return cudaGetLastError();
 }
 

@@ -77,6 +77,8 @@ cudaError_t launch_probe_detector(const TransportParams& P, int n, const float* 
                                   const int8_t* s2, const int8_t* s1, int2* seeds, int* out, cudaStream_t s);
 cudaError_t launch_probe_compton(const ComptonTable* tab, int n, float* energy, const int* mat, int2* seeds,
                                  double* costh, cudaStream_t s);
+cudaError_t launch_probe_compton_test(const ComptonTable* tab, int n, const float* energy, const int* mat,
+                                      const float* tau, const float* u, int* out, cudaStream_t stream);
 cudaError_t launch_probe_rayleigh(const RayleighRows& R, int n, const float* energy, const int* mat,
                                   const float* pmax, int2* seeds, double* costh, cudaStream_t s);
 cudaError_t launch_probe_source(const TransportParams& P, int background, int2* seeds, float3* out,

@@ -789,19 +789,19 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) transport_events_kernel(Tr
           } else {
             s0 = cold.f(kCS0);
           }
-          float tau = 0.f, s = 0.f, u = 0.f;
+          float tau = 0.f, s = 0.f, u = 0.f, num = 0.f, den = 1.f;
           double cdt1 = 0.0;
           bool accepted = false, tripped = false, candidate = false;
           for (;;) {
             for (;;) {
               if (!accepted && !tripped && !candidate) {
                 if (++trials > (uint32_t)rejections_cap<kMode>(P)) tripped = true;
-                else candidate = compton_envelope<(kMode & kModeFast) != 0>(rng, e, tau, cdt1, u);
+                else candidate = compton_envelope<(kMode & kModeFast) != 0>(rng, e, tau, cdt1, u, num, den);
               }
               if (8 * __popc(__ballot_sync(m_c, !accepted && !tripped && !candidate)) <= __popc(m_c)) break;
             }
             if (candidate) {
-              accepted = compton_shells(e, mat0, cmp, rn, s0, tau, cdt1, u, s);
+              accepted = compton_shells(e, mat0, cmp, rn, s0, tau, cdt1, u, num, den, s);
               candidate = false;
             }
             if (8 * __popc(__ballot_sync(m_c, !accepted && !tripped)) <= __popc(m_c)) break;

@@ -224,6 +224,7 @@ _SIGNATURES = {
     "mcpet_probe_rng": (C.c_int, [C.c_int, C.c_int, P, C.c_int, P, P, P]),
     "mcpet_probe_detector": (C.c_int, [P, C.c_int] + [P] * 10),
     "mcpet_probe_compton": (C.c_int, [P, C.c_int, P, P, P, P, P, P]),
+    "mcpet_probe_compton_test": (C.c_int, [P, C.c_int, P, P, P, P, P]),
     "mcpet_probe_rayleigh": (C.c_int, [P, C.c_int, P, P, P, P, P, P]),
     "mcpet_probe_source": (C.c_int, [C.c_int, C.c_int, C.c_int, P, C.c_int, P, P, P]),
     "mcpet_last_error": (C.c_char_p, []),

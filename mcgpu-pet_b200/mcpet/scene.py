@@ -587,6 +587,16 @@ def probe_compton(scene: Scene, energy, mat, seeds):
     return e_out, c_out, s_out
 
 
+def probe_compton_test(scene: Scene, energy, mat, tau, u):
+    """(early part rejects, whole test rejects) for each trial
+    (mcpet_probe_compton_test)."""
+    e, t, x = (np.ascontiguousarray(v, np.float32) for v in (energy, tau, u))
+    m = np.ascontiguousarray(mat, np.int32)
+    out = np.zeros(len(e), np.int32)
+    check(lib().mcpet_probe_compton_test(scene.handle, len(e), _ptr(e), _ptr(m), _ptr(t), _ptr(x), _ptr(out)))
+    return (out & 1) != 0, (out & 2) != 0
+
+
 def probe_rayleigh(scene: Scene, energy, mat, pmax, seeds):
     e = np.ascontiguousarray(energy, np.float32)
     m = np.ascontiguousarray(mat, np.int32)
