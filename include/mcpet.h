@@ -483,6 +483,11 @@ mcpet_status mcpet_write_outputs(const mcpet_scene* scene, const mcpet_tallies* 
 mcpet_status mcpet_probe_rng(int n, int seed_input, const int64_t* stream_ids, int ndraw,
                              int32_t* seeds_out, float* draws, double* ddraws);
 
+/* How the scene's last launch (of a run, a batch or a graph's creation) started
+ * its lanes: 1 the longest ones on warps of their own, 0 packed, -1 no launch
+ * yet. */
+mcpet_status mcpet_probe_start(const mcpet_scene* scene, int32_t* spread);
+
 /* Detector model on a fixed event list (tally_Sinogram,
  * MCGPU-PET_kernel.cu:1624-1836) on the GPU with the scene's detector and
  * sinogram geometry.  Per event: out[6*i+0]=bin or -1, +1 class (1 true, 2

@@ -544,17 +544,35 @@ double scene_decays(const mcpet_scene* sc) {
   return emitting_activity(sc) * ((double)sc->cfg.acquisition_time_ps * 1e-12) / sc->tune_scale;
 }
 
-/* Whether a launch of `decays` expected decays, at most `longest` of them in
- * one lane, starts its longest lanes on warps of their own: where their
- * chains bound the run.  A chain takes about 26 us a decay in a full warp
- * (8 us alone) and the whole GPU 0.4 ns a decay, so the chains of a packed
- * start end after the rest when a lane holds more than about 1/65000 of the
- * decays; the line is at four times that, where spreading gains whatever the
- * lanes share.  Above it a spread start is 3 times faster (1e7 decays of the
- * 9^3 cube, a lane 1/330 of them: 773 -> 253 ms); below, packed lanes share
- * voxels and scenes (58 095 decays of the cube, a lane 1/58095: 0.417 ms
- * packed, 0.432 spread; the 1e9-decay head: equal). */
-int spread_lanes(double longest, double decays) { return longest * 16384.0 > decays ? 1 : 0; }
+/* Whether a launch over the lanes of these scenes starts its longest lanes on
+ * warps of their own: where their chains bound the run.  Both quantities are
+ * those of the full acquisition, also while the autotuner runs a sample of it,
+ * so that a sample starts like the run that it stands for.  A chain takes
+ * about 26 us a decay in a full warp (8 us alone) and the whole GPU 0.4 ns a
+ * decay, so the chains of a packed start end after the rest when a lane holds
+ * more than about 1/65000 of the decays.  The line is at four times that.
+ * Packed over spread time, 48^3 cube, reference and balanced lanes, a lane
+ * 1/r of the decays:
+ *   32 hot lanes beside 1e5 others, 1e6 decays: r 1000 2.7 2.7, 4000 2.1 2.3,
+ *     8000 1.7 2.1, 16000 1.3 1.8, 32000 1.08 1.35, 58000 1.09 0.92 (2e7
+ *     decays: 3.0 2.8 to 1.30 0.93);
+ *   r lanes alike, 30 decays each: 1000 2.5 2.3, 4000 2.0 1.9, 8000 1.5 1.6,
+ *     12000 1.04 1.24, 16000 0.92 1.01, 24000 0.84 0.90, 58000 0.81 0.83 (2
+ *     decays each: 1.7 1.5 to 1.06 1.06).
+ * So far above the line a spread start is up to 3 times faster whatever the
+ * lanes (1e7 decays of the 9^3 cube, a lane 1/330 of them: 773 -> 253 ms), at
+ * the line hot lanes gain more than lanes alike lose, and below it lanes
+ * alike, the common plan, lose up to a fifth.  A run over ranges of lanes
+ * takes the whole scene's start for each range. */
+struct LaneChains {
+  double longest = 0;   /* expected decays of the longest lane */
+  double decays = 0;    /* of all lanes */
+  void add(const mcpet_scene* sc) {
+    longest = std::max(longest, sc->dev.max_lane_decays / sc->tune_scale);
+    decays += scene_decays(sc);
+  }
+  int spread() const { return longest * 16384.0 > decays ? 1 : 0; }
+};
 
 /* Kernel variant of a run: balanced lanes use the single-precision
  * rotation and decay clock (they are held to statistical parity; reference
@@ -589,7 +607,10 @@ mcpet_status launch_planned(mcpet_scene* sc, const mcpet_run_opts& o, TransportP
       return set_error(MCPET_ERR_ARG, "lowered loop caps are not available for the gradient's recording run");
     if (algorithm != kAlgorithmEvents || (mode & kTransportPrompt)) algorithm = kAlgorithmHistories;
   }
-  P.spread_lanes = spread_lanes(d.max_lane_decays, scene_decays(sc));
+  LaneChains chains;
+  chains.add(sc);
+  P.spread_lanes = algorithm == kAlgorithmHistories ? 0 : chains.spread();
+  d.last_start = P.spread_lanes;
   size_t smem = transport_dynamic_smem(P, block, algorithm);
   int bps = 0;
   CUDA_TRY(transport_occupancy(counters, algorithm, mode, block, smem, &bps));
@@ -968,16 +989,14 @@ mcpet_status setup_batch(mcpet_scene* const* scenes, int n, const mcpet_run_opts
       lanes += L.slots[(size_t)i].P.n_lanes;
     }
     L.total += lanes;
-    double longest = 0, decays = 0;
-    for (int i = j; i < j + g.count; ++i) {
-      const mcpet_scene* sc = scenes[L.scene_of[(size_t)i]];
-      longest = std::max(longest, sc->dev.max_lane_decays);
-      decays += scene_decays(sc);
-    }
+    LaneChains chains;
+    for (int i = j; i < j + g.count; ++i) chains.add(scenes[L.scene_of[(size_t)i]]);
+    const int spread = chains.spread();
+    for (int i = j; i < j + g.count; ++i) scenes[L.scene_of[(size_t)i]]->dev.last_start = spread;
     if (g.solo) {
       const int k = L.scene_of[(size_t)j];
       g.P = alone[(size_t)k];
-      g.P.spread_lanes = spread_lanes(longest, decays);
+      g.P.spread_lanes = spread;
       g.T = L.slots[(size_t)j].T;
       g.O = L.slots[(size_t)j].O;
       g.mode = run_mode(scenes[k], o) | kTransportChained;
@@ -988,7 +1007,7 @@ mcpet_status setup_batch(mcpet_scene* const* scenes, int n, const mcpet_run_opts
     }
     g.P = L.slots[(size_t)j].P;
     g.P.n_lanes = lanes;
-    g.P.spread_lanes = spread_lanes(longest, decays);
+    g.P.spread_lanes = spread;
     g.P.n_emitters = 0;
     g.P.max_shells = max_shells;
     /* the launch's shared layout holds the prompt-gamma fields when any of
@@ -2206,6 +2225,7 @@ mcpet_status mcpet_run_device_noalloc(mcpet_scene* sc, const float* activity_dev
   if (o.blocks_per_sm > 0 && o.blocks_per_sm < bps) bps = o.blocks_per_sm;
   const int grid = d.sm_count * bps;
   d.last_run_noalloc = true;
+  d.last_start = 0;   /* its plan is in voxel order, not by work: packed */
   CUDA_TRY(launch_transport_noalloc(P, device_tables(sc), O, activity_device, o.lane_mode, tpb, hpl, d.sm_count,
                                     counters, mode, grid, block, smem, st));
   return MCPET_OK;
@@ -2256,6 +2276,12 @@ mcpet_status probe_device() {
 }  // namespace
 
 extern "C" {
+
+mcpet_status mcpet_probe_start(const mcpet_scene* sc, int32_t* spread) {
+  if (!sc || !spread) return set_error(MCPET_ERR_ARG, "invalid probe arguments");
+  *spread = sc->dev.last_start;
+  return MCPET_OK;
+}
 
 mcpet_status mcpet_probe_rng(int n, int seed_input, const int64_t* stream_ids, int ndraw, int32_t* seeds_out,
                              float* draws, double* ddraws) {

@@ -57,6 +57,7 @@ struct mcpet_scene {
     int n_emitters = 0;
     uint64_t n_lanes = 0;
     double max_lane_decays = 0;   /* expected decays of the plan's longest lane */
+    int last_start = -1;          /* the last launch's spread_lanes; -1 before the first */
     std::string plan_key;
     /* run scratch owned by the scene (host-buffer runs) */
     int* trues = nullptr;

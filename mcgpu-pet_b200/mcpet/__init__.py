@@ -7,12 +7,12 @@ from ._abi import (ALGORITHM_AUTO, ALGORITHM_EVENTS, ALGORITHM_HISTORIES, LANES_
                    MAX_MATERIALS, McpetError, EXPORTED, LIB_PATH, lib)
 from .scene import (PSF_DTYPE, BatchGraph, RunOptions, RunResult, Scene, autotune, device_tallies_for,
                     probe_compton, probe_compton_test, probe_detector, probe_rayleigh, probe_rng, probe_source,
-                    read_config)
+                    probe_start, read_config)
 
 __all__ = [
     "ALGORITHM_AUTO", "ALGORITHM_EVENTS", "ALGORITHM_HISTORIES", "LANES_BALANCED", "LANES_REFERENCE", "MAX_MATERIALS", "McpetError", "EXPORTED", "LIB_PATH", "lib", "PSF_DTYPE",
     "BatchGraph", "RunOptions", "RunResult", "Scene", "autotune", "device_tallies_for", "probe_compton", "probe_compton_test", "probe_detector", "probe_rayleigh", "probe_rng",
-    "probe_source", "read_config",
+    "probe_source", "probe_start", "read_config",
 ]
 
 

@@ -222,6 +222,7 @@ _SIGNATURES = {
     "mcpet_batch_graph_destroy": (None, [P]),
     "mcpet_write_outputs": (C.c_int, [P, C.POINTER(Tallies), C.c_char_p, C.c_int, C.c_double]),
     "mcpet_probe_rng": (C.c_int, [C.c_int, C.c_int, P, C.c_int, P, P, P]),
+    "mcpet_probe_start": (C.c_int, [P, P]),
     "mcpet_probe_detector": (C.c_int, [P, C.c_int] + [P] * 10),
     "mcpet_probe_compton": (C.c_int, [P, C.c_int, P, P, P, P, P, P]),
     "mcpet_probe_compton_test": (C.c_int, [P, C.c_int, P, P, P, P, P]),

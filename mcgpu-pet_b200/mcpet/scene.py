@@ -562,6 +562,14 @@ def probe_rng(seed: int, stream_ids, ndraw: int = 8):
     return seeds, f, d
 
 
+def probe_start(scene: Scene) -> int:
+    """1 when the scene's last launch started its longest lanes on warps of
+    their own, 0 packed, -1 before the first (mcpet_probe_start)."""
+    out = np.zeros(1, np.int32)
+    check(lib().mcpet_probe_start(scene.handle, _ptr(out)))
+    return int(out[0])
+
+
 def probe_detector(scene: Scene, ev: dict) -> np.ndarray:
     n = len(ev["e2"])
     a = {k: np.ascontiguousarray(ev[k], dtype=(np.int8 if k.startswith("st") else

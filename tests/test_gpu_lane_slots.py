@@ -81,3 +81,27 @@ def test_batch_equals_runs_alone(workdir, count):
             assert x.total_histories == y.total_histories and x.detected == y.detected
             for k in ("trues", "scatter", "image_trues", "image_scatter", "spectrum"):
                 np.testing.assert_array_equal(getattr(x, k), getattr(y, k), err_msg=k)
+
+
+@pytest.mark.parametrize("batch", [False, True], ids=["one", "batch"])
+def test_autotuner_samples_start_like_the_run(workdir, batch):
+    """8000 lanes of 50 decays: each 1/8000 of the decays (1/16000 of two
+    scenes'), above the line of a spread start (1/16384) in the run and in a
+    sample of a fifth of it."""
+    shape = (20, 20, 20)
+    mat, rho = np.full(shape, 2, np.int32), np.ones(shape, np.float32)
+    act = np.full(shape, 50.0, np.float32)
+    o = mcpet.RunOptions(lane_mode=mcpet.LANES_REFERENCE)
+    sc = [scenes.scene_from_arrays(workdir, mat, rho, act, (0.5, 0.5, 0.5), threads_per_block=1, seed=21 + k)
+          for k in range(2 if batch else 1)]
+    tal = [mcpet.device_tallies_for(s) for s in sc]
+    if batch:
+        mcpet.Scene.run_batch_device(sc, tal, o)
+    else:
+        sc[0].run_device(tal[0], o)
+    assert [mcpet.probe_start(s) for s in sc] == [1] * len(sc)
+    _, info = mcpet.autotune(sc, tal, o, sample_decays=8.0e4 * len(sc))
+    assert abs(info["sample_fraction"] - 0.2) < 1e-6
+    assert [mcpet.probe_start(s) for s in sc] == [1] * len(sc)
+    for s in sc:
+        s.close()
