@@ -1,11 +1,14 @@
 """The event kernel's first lanes and its queue.
 
-The first lanes are dealt to the warps one by one when one lane is long, the
-rest come from the work queue.  The tallies do not depend on it: a grid of one
-warp per SM gives the same ones, to the last record, as the full grid with a
-thread for every lane, at lane counts around the threads and twice them; and
-both agree with the history loop (same draws; its multiply-adds may contract
-otherwise, which parts a history in a million)."""
+Where one lane is long against the launch (more than 1/16384 of its decays) the
+first lanes are dealt to the warps one by one, longest first, and the rest come
+from the work queue; elsewhere the queue deals every lane.  The tallies do not
+depend on it: a grid of one warp per SM gives the same ones, to the last
+record, as the full grid, at lane counts around the threads of the small grid
+and above those of any grid; a scene that starts spread alone gives the same
+ones packed in a batch; and all agree with the history loop (same draws; its
+multiply-adds may contract otherwise, which parts a history in a million).
+Each test states which start its scene takes and checks it."""
 import numpy as np
 import pytest
 
@@ -15,47 +18,56 @@ import scenes
 
 pytestmark = pytest.mark.gpu
 THREADS = 32          # a block of one warp, one block per SM
+SPREAD, PACKED = 1, 0
 
 
 def _lanes(which):
     import torch
     t = THREADS * torch.cuda.get_device_properties(0).multi_processor_count
-    return {"1": 1, "31": 31, "33": 33, "T-1": t - 1, "T": t, "T+1": t + 1, "2T-1": 2 * t - 1, "2T": 2 * t,
-            "2T+1": 2 * t + 1, "3T+5": 3 * t + 5}[which]
+    return {"1": 1, "31": 31, "33": 33, "T-1": t - 1, "T": t, "T+1": t + 1, "3T+5": 3 * t + 5,
+            "26^3": 26 ** 3,            # just below the line when all lanes are alike
+            "68^3": 68 ** 3}[which]     # more than 2048 threads on each of 148 SMs
 
 
-def _scene(workdir, n, hot, **kw):
-    """A water block with one lane in each of its first n voxels (about 3
-    decays each; the hot one holds most of the run's decays, which spreads
-    the first lanes over the warps)."""
-    shape = (26, 26, 26)
+def _scene(workdir, n, activity, **kw):
+    """A water cube with one lane in each of its first n voxels, about 3
+    decays each.  alike: the same in all; uneven: 1 to 5; hot: uneven, and one
+    voxel among them with 400."""
+    side = 26 if n <= 26 ** 3 else 68
+    shape = (side,) * 3
     mat, rho = np.full(shape, 2, np.int32), np.ones(shape, np.float32)
     act = np.zeros(shape, np.float32)
-    act.ravel()[:n] = np.random.default_rng(n).uniform(1, 5, n)
-    if hot:
-        act.ravel()[n // 2] = 400.0 + n / 16
-    return scenes.scene_from_arrays(workdir, mat, rho, act, (0.4, 0.4, 0.4), threads_per_block=1, **kw)
+    act.ravel()[:n] = 3.0 if activity == "alike" else np.random.default_rng(n).uniform(1, 5, n)
+    if activity == "hot":
+        act.ravel()[n // 2] = 400.0
+    if kw.get("voxel_dose"):
+        kw["dose_roi"] = (1, side) * 3
+    return scenes.scene_from_arrays(workdir, mat, rho, act, (10.4 / side,) * 3, threads_per_block=1, **kw)
 
 
 KINDS = {
     "sinogram": dict(),
-    "psf": dict(tally_psf_sinogram=0, psf_size=200000),
-    "dose": dict(material_dose=True, voxel_dose=True, dose_roi=(1, 26, 1, 26, 1, 26)),
+    "psf": dict(tally_psf_sinogram=0, psf_size=1000000),
+    "dose": dict(material_dose=True, voxel_dose=True),
 }
+# lanes, activity, start: fewer than 16384 lanes spread whatever their activity
+CASES = [(c, "uneven", SPREAD) for c in ("1", "31", "33", "T-1", "T", "T+1", "3T+5")]
+CASES += [(c, "hot", SPREAD) for c in ("33", "T", "3T+5", "68^3")]
+CASES += [("26^3", "alike", PACKED), ("68^3", "alike", PACKED)]
+RUNS = [("sinogram",) + c for c in CASES]
+RUNS += [(k,) + c for k in ("psf", "dose") for c in CASES if c[0] in ("T+1", "68^3") or c[2] == PACKED]
 
 
-@pytest.mark.parametrize("kind", sorted(KINDS))
-@pytest.mark.parametrize("hot", [False, True], ids=["even", "hot"])
 @pytest.mark.parametrize("lanes", [mcpet.LANES_REFERENCE, mcpet.LANES_BALANCED], ids=["reference", "balanced"])
-@pytest.mark.parametrize("count", ["1", "31", "33", "T-1", "T", "T+1", "2T-1", "2T", "2T+1", "3T+5"])
-def test_tallies_do_not_depend_on_the_lanes_place(workdir, count, lanes, hot, kind):
-    if kind != "sinogram" and count not in ("33", "T+1", "3T+5"):
-        pytest.skip("the other tallies at three counts")
-    with _scene(workdir, _lanes(count), hot, **KINDS[kind]) as sc:
+@pytest.mark.parametrize("kind, count, activity, start", RUNS, ids=["-".join(r[:3]) for r in RUNS])
+def test_tallies_do_not_depend_on_the_lanes_place(workdir, kind, count, activity, start, lanes):
+    with _scene(workdir, _lanes(count), activity, **KINDS[kind]) as sc:
         o = dict(lane_mode=lanes, histories_per_lane=1 << 20)
         assert sc.lane_plan(lanes, 1 << 20)["total_lanes"] == _lanes(count)
         a = sc.run(mcpet.RunOptions(block_threads=THREADS, blocks_per_sm=1, **o))
+        assert mcpet.probe_start(sc) == start
         b = sc.run(mcpet.RunOptions(**o))
+        assert mcpet.probe_start(sc) == start
         c = sc.run(mcpet.RunOptions(algorithm=mcpet.ALGORITHM_HISTORIES, **o))
         assert a.total_histories == b.total_histories == c.total_histories and a.detected == b.detected
         for k in ("trues", "scatter", "image_trues", "image_scatter", "spectrum", "material_dose", "voxel_dose"):
@@ -70,13 +82,24 @@ def test_tallies_do_not_depend_on_the_lanes_place(workdir, count, lanes, hot, ki
             np.testing.assert_array_equal(scenes.psf_records(a.psf), scenes.psf_records(b.psf))
 
 
-@pytest.mark.parametrize("count", ["33", "T+1", "3T+5"])
-def test_batch_equals_runs_alone(workdir, count):
-    """Two scenes of different lane counts in one launch."""
-    o = mcpet.RunOptions(lane_mode=mcpet.LANES_REFERENCE, block_threads=THREADS, blocks_per_sm=1)
-    with _scene(workdir, _lanes(count), False, seed=11) as a, _scene(workdir, 40, True, seed=12) as b:
+@pytest.mark.parametrize("lanes", [mcpet.LANES_REFERENCE, mcpet.LANES_BALANCED], ids=["reference", "balanced"])
+@pytest.mark.parametrize("first, second, starts", [
+    (("33", "uneven"), ("33", "hot"), (SPREAD, SPREAD, SPREAD)),
+    (("T+1", "uneven"), ("33", "hot"), (SPREAD, SPREAD, SPREAD)),
+    (("33", "uneven"), ("68^3", "alike"), (SPREAD, PACKED, PACKED)),
+    (("T+1", "uneven"), ("68^3", "alike"), (SPREAD, PACKED, PACKED)),
+    (("T", "hot"), ("68^3", "hot"), (SPREAD, SPREAD, SPREAD)),
+], ids=lambda v: "-".join(map(str, v)))
+def test_batch_equals_runs_alone(workdir, first, second, starts, lanes):
+    """Two scenes in one launch, which starts as its lanes together ask for:
+    a scene that spreads alone is packed beside many lanes."""
+    o = mcpet.RunOptions(lane_mode=lanes, histories_per_lane=1 << 20)
+    with _scene(workdir, _lanes(first[0]), first[1], seed=11) as a, \
+            _scene(workdir, _lanes(second[0]), second[1], seed=12) as b:
         alone = [s.run(o) for s in (a, b)]
+        assert (mcpet.probe_start(a), mcpet.probe_start(b)) == starts[:2]
         both = mcpet.Scene.run_batch([a, b], o)
+        assert mcpet.probe_start(a) == mcpet.probe_start(b) == starts[2]
         for x, y in zip(alone, both):
             assert x.total_histories == y.total_histories and x.detected == y.detected
             for k in ("trues", "scatter", "image_trues", "image_scatter", "spectrum"):
