@@ -24,6 +24,10 @@ Arms:
                     no part of this library is loaded) on the same fixed
                     voxel sample of the workload in every step.
 
+Where the reference builds under oracle/_ref are missing (its sources are
+needed to make them) the reference arm prints its "unavailable" line, and the
+default arm leaves ref_cuda and cpu_baseline out and says why.
+
 Multi-GPU: one process per GPU (torchrun); every rank runs an independent
 replica with its own seed (the transport has no exchange step); value = all
 detected coincidences / max rank time.
@@ -192,12 +196,27 @@ class ReferenceCPU:
                 f"load_material and its MCGPU-PET_kernel.cu compiled for the host with OpenMP)")
 
 
+def reference_unavailable(*libs):
+    """Why the reference cannot run: the builds under oracle/_ref that are
+    missing; None when all are there."""
+    sys.path.insert(0, os.path.join(ROOT, "tests"))
+    import refbind
+    missing = [n for n in libs if not refbind.available(n)]
+    if not missing:
+        return None
+    return f"reference build missing: {', '.join(missing)} (make -C oracle/ref, where the reference sources are present)"
+
+
 CPU_SAMPLE_DECAYS = 6.0e7     # 6 % of the head workload per CPU step (~5 s on 16 host threads)
 
 
 def run_reference_arm(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
+        return 0
+    why = reference_unavailable("libref_prog.so", "libref_cpu.so")
+    if why:
+        print(json.dumps({"impl": "reference", "unavailable": why}))
         return 0
     with tempfile.TemporaryDirectory() as tmp:
         ref = ReferenceCPU(write_workload_files(tmp, args.emissions), tmp)
@@ -680,13 +699,15 @@ def main():
         beds = measure_beds(args.beds, tmp)
 
     ref_cuda = None
-    if rank == 0 and world == 1 and not args.no_ref_cuda and args.scanner == "head":
+    no_ref_cuda, no_ref_cpu = reference_unavailable("libref_prog.so"), \
+        reference_unavailable("libref_prog.so", "libref_cpu.so")
+    if rank == 0 and world == 1 and not args.no_ref_cuda and args.scanner == "head" and not no_ref_cuda:
         ref_cuda = measure_reference_cuda(tmp, args.emissions)
         ref_cuda["this_library_kernel_ms"] = avg_kernel_ms
         ref_cuda["kernel_time_ratio"] = ref_cuda["kernel_ms"] / avg_kernel_ms
 
     cpu = None
-    if rank == 0 and world == 1 and not args.no_cpu_baseline:
+    if rank == 0 and world == 1 and not args.no_cpu_baseline and not no_ref_cpu:
         ref = ReferenceCPU(write_workload_files(tmp, args.emissions), tmp)
         blocks = ref.sample(args.cpu_sample_decays)
         ref.run(ref.sample(args.cpu_sample_decays / 25))          # warm-up
@@ -698,7 +719,7 @@ def main():
         line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": elapsed_ms / args.steps, "higher_is_better": True,
                 "scaling": "weak", "vs_baseline": None, "dtype": "f32",
-                "data": "synthetic (seeded head phantom; tissue densities on the reference's own air/water material tables)",
+                "data": "synthetic (seeded head phantom; tissue densities on the staged air/water material tables)",
                 "config": bench_config(args.emissions, world),
                 "impl_config": {"lanes": args.lanes, "algorithm": args.algorithm,
                                 "block_threads": args.block_threads or "auto",
@@ -706,6 +727,8 @@ def main():
                 "run": {"coincidences_per_step": total / args.steps / world, "histories_last_step": hist,
                         "guard_trips": guard},
                 "roofline": roof, "cpu_baseline": cpu, "e2e": e2e, "gpu_launches": args.steps, "clocks": clocks}
+        if no_ref_cuda or no_ref_cpu:
+            line["reference_unavailable"] = no_ref_cpu or no_ref_cuda
         if ref_cuda is not None:
             line["ref_cuda"] = ref_cuda
         if gradient is not None:

@@ -39,3 +39,25 @@ def test_reference_arm_json_line_and_libraries():
     assert not ours, ours
     names = {os.path.basename(l) for l in libs}
     assert {"libref_prog.so", "libref_cpu.so"} <= names
+
+
+_NO_REF = """
+import sys
+sys.path[:0] = [{root!r}, {tests!r}]
+import refbind
+refbind.REF_DIR = {empty!r}
+sys.argv = ["bench.py", "--impl", "reference", "--steps", "1", "--warmup", "0"]
+import bench
+sys.exit(bench.main())
+"""
+
+
+def test_reference_arm_says_that_it_is_unavailable(tmp_path):
+    """Without the reference builds the arm prints one line with the reason
+    and exits 0."""
+    code = _NO_REF.format(root=ROOT, tests=os.path.join(ROOT, "tests"), empty=str(tmp_path))
+    out = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0, out.stderr[-2000:]
+    lines = [json.loads(l) for l in out.stdout.splitlines() if l.startswith("{")]
+    assert len(lines) == 1 and lines[0]["impl"] == "reference"
+    assert "libref_prog.so" in lines[0]["unavailable"] and "libref_cpu.so" in lines[0]["unavailable"]
