@@ -446,7 +446,8 @@ void mcpet_batch_graph_destroy(mcpet_batch_graph* graph);
  * before any stream capture.  The address is kept for the life of the
  * device's context: do not use this entry point across a cudaDeviceReset.
  * Lanes are laid out in voxel order: with MCPET_LANES_REFERENCE the results
- * equal mcpet_run_device's; with balanced lanes and histories_per_lane <= 0
+ * equal mcpet_run_device's, but no lane starts on a warp of its own, so a
+ * phantom with a few far hotter voxels takes longer; with balanced lanes and histories_per_lane <= 0
  * the automatic lane size is computed on the device from activity_device.
  * A plan whose RANECU stream ids would reach 2^31 (the reference's 31-bit
  * thread ids) runs nothing and counts one guard trip.  Guard trips (that

@@ -560,7 +560,7 @@ double scene_decays(const mcpet_scene* sc) {
  *     12000 1.04 1.24, 16000 0.92 1.01, 24000 0.84 0.90, 58000 0.81 0.83 (2
  *     decays each: 1.7 1.5 to 1.06 1.06).
  * So far above the line a spread start is up to 3 times faster whatever the
- * lanes (1e7 decays of the 9^3 cube, a lane 1/330 of them: 773 -> 253 ms), at
+ * lanes (1e7 decays of the 9^3 cube, a lane 1/330 of them: 800 -> 253 ms), at
  * the line hot lanes gain more than lanes alike lose, and below it lanes
  * alike, the common plan, lose up to a fifth.  A run over ranges of lanes
  * takes the whole scene's start for each range. */

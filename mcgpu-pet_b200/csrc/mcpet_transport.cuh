@@ -80,15 +80,18 @@ __device__ __forceinline__ uint64_t claim_lane(unsigned long long* cursor) {
 }
 
 /* The lanes a grid starts with when they are spread (TransportParams::
- * spread_lanes): the lane of rank r -- plans are ordered by decreasing work --
- * goes to warp r mod W of the grid's W warps, warps counted across the blocks
- * first, so that the longest lanes start on warps of their own on different
- * SMs; later ones come from the work queue, after the first gridDim *
- * blockDim.  A lane is one serial chain of decays, and in a full warp it
- * waits for the rounds of 31 others: 25.8 us a decay with 32 of the hot
- * lanes of a 9^3 cube to a warp, 8.3 us with one (1e7 decays, 96 lanes of
- * 30458 decays each: 787 -> 253 ms).  Elsewhere the queue deals every lane,
- * in groups of consecutive ones that share voxels and scenes. */
+ * spread_lanes): the lane of rank r -- a scene's plan is ordered by decreasing
+ * work; in a batch each scene's lanes follow one another, the scene with the
+ * longest lane first -- goes to warp r mod W of the grid's W warps, warps
+ * counted across the blocks first, so that the longest lanes start on warps of
+ * their own on different SMs; later ones come from the work queue, after the
+ * first gridDim * blockDim (where there are more, the threads beside a long
+ * lane claim them and it shares its warp until the queue is empty).  A lane is
+ * one serial chain of decays, and in a full warp it waits for the rounds of 31
+ * others: 25.8 us a decay with 32 of the hot lanes of a 9^3 cube to a warp,
+ * 8.3 us with one (1e7 decays, 96 lanes of 30458 decays each: 800 -> 253 ms,
+ * in turn on one GPU).  Elsewhere the queue deals every lane, in groups of
+ * consecutive ones that share voxels and scenes. */
 __device__ __forceinline__ uint64_t initial_lane() {
   const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
   return (threadIdx.x & 31) * warps + (uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
